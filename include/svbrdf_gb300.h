@@ -182,7 +182,7 @@ typedef struct svbrdf_batch_config {
 /* Workspace of svbrdf_batched_step: the int32 at byte offset 4 is a device error word,
  * 0 while healthy. A pipelined launch that waited too long for its copies or consumers
  * stores a non-zero code there (1: copy never landed, 2: consumers stalled, 3: drain
- * timeout), skips the rest of its work and returns; the caller reads the word after
+ * timeout, 4: an iteration of a cooperative launch never ended in some CTA), skips the rest of its work and returns; the caller reads the word after
  * synchronising and treats non-zero as a failed step. */
 #define SVBRDF_WORKSPACE_ERROR_OFFSET 4
 

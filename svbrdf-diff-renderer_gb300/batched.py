@@ -56,8 +56,8 @@ class BatchedOptim:
 
     With ``optim_light`` every material's light power is optimised with its maps, as
     ``SvbrdfOptim.optim(..., optim_light=True)`` does (src/svbrdf.py:48-50, 58-59); the
-    current values are ``light_pow(i)``. That needs the texel-pair kernels (variants 2 and 3),
-    and each iteration is then its own launch. With ``adopt_maps`` a material's ``init``
+    current values are ``light_pow(i)``. That needs the texel-pair kernels (variants 2 and 3):
+    variant 2 then runs up to 32 iterations per cooperative launch, variant 3 one. With ``adopt_maps`` a material's ``init``
     tensor that is already a contiguous FP32 tensor on the device becomes the optimised
     maps in place instead of being copied."""
 
@@ -112,7 +112,9 @@ class BatchedOptim:
         return sum(H * W * (216 + 12 * V) for H, W, V, _ in self.meta)
 
     def launches(self, iters: int) -> int:
-        """Kernel launches ``iters`` iterations take with this plan's variant."""
+        """Kernel launches ``iters`` iterations take with this plan's variant. With a learnable light
+        every iteration counts as one, although the texel-pair kernel runs up to FUSE_MAX of them
+        in one cooperative launch where the device holds its whole grid at once."""
         return -(-iters // FUSE_MAX) if self.config.variant >= 3 and not self.optim_light else iters
 
     def light_pow(self, i: int) -> torch.Tensor:

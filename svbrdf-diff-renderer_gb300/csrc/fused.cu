@@ -55,16 +55,34 @@ AdamScalars make_adam(int step, float lr, float beta1, float beta2, float eps) {
   return s;
 }
 
-__device__ __forceinline__ AdamScalars device_adam(const AdamHyper& h, int step) {
-  const double bc1 = 1.0 - pow((double)h.beta1, (double)step);
-  const double bc2 = 1.0 - pow((double)h.beta2, (double)step);
-  AdamScalars s;
+// b^n by repeated squaring: at most 2 log2(n) double multiplications, each rounding once, so
+// about 30 units of 2^-53 at n = 10^5, far below the FP32 rounding of the scalars it feeds.
+__device__ __forceinline__ double ipow(double b, int n) {
+  double r = 1.0;
+  for (unsigned e = (unsigned)n; e; e >>= 1) {
+    if (e & 1u) r *= b;
+    b *= b;
+  }
+  return r;
+}
+
+// The two bias corrections are independent chains of double-precision operations, which this
+// GPU issues at 1/64 of its FP32 rate: adam_first and adam_second fill one half of the scalars
+// each, so that the pipelined kernels can run them in two warps side by side.
+__device__ __forceinline__ void adam_first(const AdamHyper& h, int step, AdamScalars& s) {
   s.one_minus_b1 = (float)(1.0 - (double)h.beta1);
+  s.eps = h.eps;
+  s.neg_step_size = (float)(-(double)h.lr / (1.0 - ipow((double)h.beta1, step)));
+}
+__device__ __forceinline__ void adam_second(const AdamHyper& h, int step, AdamScalars& s) {
   s.b2 = h.beta2;
   s.one_minus_b2 = (float)(1.0 - (double)h.beta2);
-  s.inv_bc2_sqrt = (float)(1.0 / sqrt(bc2));
-  s.eps = h.eps;
-  s.neg_step_size = (float)(-(double)h.lr / bc1);
+  s.inv_bc2_sqrt = (float)(1.0 / sqrt(1.0 - ipow((double)h.beta2, step)));
+}
+__device__ __forceinline__ AdamScalars device_adam(const AdamHyper& h, int step) {
+  AdamScalars s;
+  adam_first(h, step, s);
+  adam_second(h, step, s);
   return s;
 }
 
@@ -240,7 +258,7 @@ __device__ __forceinline__ void texel_rc(int idx, const MatDesc& md, int& i, int
 // losses are deterministic; the last CTA reads one value per tile and iteration instead of
 // one per warp (15x fewer), in parallel across its warps.
 template <int NT>
-__device__ __forceinline__ void batched_finish(const char* plan, const PlanHeader* hdr, const MatDesc* mats,
+__device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeader* hdr, const MatDesc* mats,
                                                const float* partial, int per_tile, float* loss_hist, int hist_len,
                                                int step, int* step_counter, unsigned* counter, int* s_flag,
                                                int nwarps, int iters = 1, const float* lpart = nullptr,
@@ -278,7 +296,7 @@ __device__ __forceinline__ void batched_finish(const char* plan, const PlanHeade
     *s_flag = (prev == gridDim.x - 1) ? 1 : 0;
   }
   __syncthreads();
-  if (!*s_flag) return;
+  if (!*s_flag) return false;
   __threadfence();
   const int* mat_tiles = (const int*)(plan + hdr->off_mat_tiles);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -326,6 +344,36 @@ __device__ __forceinline__ void batched_finish(const char* plan, const PlanHeade
     *step_counter = step;
     *counter = 0u;
   }
+  return true;
+}
+
+// End of an iteration inside a cooperative launch: the last CTA, whose writes in batched_finish
+// come first, publishes the iteration's number in ws[kWsIteration]; the others wait for it. The
+// wait is bounded (about a second of polls); false in every thread if it ran out.
+__device__ __forceinline__ bool batched_next_iteration(bool last, unsigned* ws, unsigned number, int* s_flag) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    if (last) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ws + kWsIteration), "r"(number) : "memory");
+    } else {
+      for (uint32_t it = 0;; ++it) {
+        unsigned now;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(ws + kWsIteration) : "memory");
+        if (now == number) break;
+        if (it >= (1u << 21) || *(volatile unsigned*)(ws + kWsError)) {
+          atomicCAS((int*)(ws + kWsError), 0, (int)kDevTimeoutGrid);
+          ok = 0;
+          break;
+        }
+      }
+      __threadfence();
+    }
+    *s_flag = ok;
+  }
+  __syncthreads();
+  return *s_flag != 0;
 }
 
 // Light-power gradient partial of one warp's texels of one tile: lanes' values summed in a
@@ -778,6 +826,12 @@ batched_tma_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restri
 // Waits, error recording and draining follow variant 1. GEN instantiations also carry the
 // general (light off the camera) path; plans whose views are all co-located launch the
 // instantiation without it, which keeps its registers for the co-located loop.
+//
+// A plan with a learnable light steps it between iterations, which every CTA then needs. Up to
+// kFuseMax iterations run in one cooperative launch: at the end of each, the last CTA to arrive
+// reduces and steps the light (batched_finish) and the others wait for it. One launch per
+// iteration paid its start (launch, plan and Adam scalars, an empty ring) and its drain each
+// time: on one 512^2 material with 9 views 33 us per iteration; the cooperative form LIGHT_US us.
 constexpr int kPairSlotPlanes = 9;
 constexpr int kPairChunkViews = 3;
 constexpr size_t kPairRingBudget = 216 * 1024;
@@ -813,7 +867,7 @@ struct __align__(16) PairSlotRec {
   float* m2;
   float* unused;
   int tile, first, W, H;        // ... tile id and first texel
-  int V, all_coloc, pad0, pad1;
+  int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
   float P[4];                   // light power
 };
@@ -821,8 +875,8 @@ struct __align__(16) PairSlotRec {
 template <int LOSS, int NCW, bool GEN>
 __global__ void __launch_bounds__((NCW + 1) * 32, NCW <= kPairTwoCtaNcw ? 2 : 1)
 batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restrict__ step_counter,
-                    float* __restrict__ loss_hist, int hist_len, float* __restrict__ warp_loss, unsigned* ws,
-                    float* __restrict__ lpart) {
+                    float* __restrict__ loss_hist, int hist_len, int iters, float* __restrict__ warp_loss,
+                    unsigned* ws, float* __restrict__ lpart) {
   constexpr int NT = NCW * 32;
   constexpr int TT = 2 * NT;                  // texels per tile
   constexpr int SLOT = kPairSlotPlanes * TT;  // floats per ring slot
@@ -832,8 +886,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   __shared__ MatDesc s_prod_md;            // the producer's current material ...
   __shared__ View s_prod_views[kMaxViews];  // ... its views
   __shared__ float s_prod_pow[4];           // ... and light power
-  __shared__ AdamScalars s_adam;
-  __shared__ int s_step;
+  __shared__ AdamScalars s_adam[kFuseMax];
   __shared__ int s_last;
 
   const PlanHeader* hdr = (const PlanHeader*)plan;
@@ -841,6 +894,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   const View* views = (const View*)(plan + hdr->off_views);
   const int* cta_off = (const int*)(plan + hdr->off_cta);
   const int R = hdr->ring_slots;
+  const int n_tiles = hdr->n_tiles;
   PairSlotRec* recs = reinterpret_cast<PairSlotRec*>(ring + (size_t)R * SLOT);
   int* err = (int*)(ws + kWsError);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -851,283 +905,310 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       mbar_init(smem_u32(&empty_bar[s]), NCW);
     }
     fence_mbar_init();
-    s_step = *step_counter + 1;
-    s_adam = device_adam(hyper, s_step);
   }
+  const int step0 = *step_counter;  // steps step0 + 1 .. step0 + iters
+  if (warp == 1 && lane < iters) adam_first(hyper, step0 + 1 + lane, s_adam[lane]);
+  if (warp == 2 && lane < iters) adam_second(hyper, step0 + 1 + lane, s_adam[lane]);
+  const unsigned number0 = __ldcg(ws + kWsIteration);
   __syncthreads();
   const int k0 = cta_off[blockIdx.x], k1 = cta_off[blockIdx.x + 1];
   const uint32_t ring_base = smem_u32(ring);
+  // the ring goes on through a launch's iterations: the producer's and the consumers' cursors
+  int slot = 0;
+  uint32_t phase = 0;
+  long long issued = 0;
+  bool ok = true;
+  RingCursor rc{0, 0u, true};
 
-  if (warp == NCW) {
-    // ------------------------------------------------------------ producer (the whole warp)
-    // Lane 0 fills the slot's record and posts the chunk's bytes on its full barrier (a
-    // release that publishes the record); lanes 0 .. nplanes-1 then issue one plane copy
-    // each. The next tile's entry is loaded one tile ahead and a material's fields and
-    // views only when the material changes.
-    const int4* seq = (const int4*)(plan + hdr->off_seq);
-    int slot = 0;
-    uint32_t phase = 0;
-    long long issued = 0;
-    bool ok = true;
-    int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
-    int cur = -1;
-    for (int k = k0; k < k1 && ok; ++k) {
-      const int4 sq = sq_next;
-      if (k + 1 < k1) sq_next = seq[k + 1];
-      if (sq.y != cur) {
-        cur = sq.y;
-        __syncwarp();
-        const MatDesc& m = mats[cur];
-        if (lane == 0) s_prod_md = m;
-        if (lane < 3) s_prod_pow[lane] = m.lpow[lane];
-        for (int v = lane; v < m.V; v += 32) s_prod_views[v] = views[m.view_off + v];
-        __syncwarp();
-      }
-      const MatDesc& md = s_prod_md;
-      const int T = md.H * md.W, V = md.V;
-      const int first = sq.z;
-      const uint32_t bytes = (uint32_t)min(TT, T - first) * 4u;
-      const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
-      for (int q = 0; q < nt + 4; ++q) {
-        if (issued >= R) {
-          ok = __all_sync(0xffffffffu, wait_phase(smem_u32(&empty_bar[slot]), phase ^ 1u, err, kDevTimeoutEmpty));
-          if (!ok) break;
+  for (int it = 0; it < iters; ++it) {
+    if (warp == NCW) {
+      // ------------------------------------------------------------ producer (the whole warp)
+      // Lane 0 fills the slot's record and posts the chunk's bytes on its full barrier (a
+      // release that publishes the record); lanes 0 .. nplanes-1 then issue one plane copy
+      // each. The next tile's entry is loaded one tile ahead and a material's fields and
+      // views only when the material changes.
+      const int4* seq = (const int4*)(plan + hdr->off_seq);
+      const bool was_ok = ok;
+      int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
+      int cur = -1;
+      for (int k = k0; k < k1 && ok; ++k) {
+        const int4 sq = sq_next;
+        if (k + 1 < n_tiles) sq_next = seq[k + 1];
+        if (sq.y != cur) {
+          cur = sq.y;
+          __syncwarp();
+          const MatDesc& m = mats[cur];
+          if (lane == 0) s_prod_md = m;
+          if (lane < 3) s_prod_pow[lane] = __ldcg(m.lpow + lane);  // another CTA may have stepped it
+          for (int v = lane; v < m.V; v += 32) s_prod_views[v] = views[m.view_off + v];
+          __syncwarp();
         }
-        const float* base;
-        int plane0, nplanes;
-        if (q == 0 || q == nt + 1) { base = md.tex; plane0 = 0; nplanes = 9; }
-        else if (q <= nt) {
-          base = md.tgt;
-          plane0 = 3 * kPairChunkViews * (q - 1);
-          nplanes = min(3 * kPairChunkViews, 3 * V - plane0);
-        }
-        else if (q == nt + 2) { base = md.m1; plane0 = 0; nplanes = 9; }
-        else { base = md.m2; plane0 = 0; nplanes = 9; }
-        const uint32_t fb = smem_u32(&full_bar[slot]);
-        if (lane == 0) {
-          PairSlotRec& r = recs[slot];
-          if (q == 0 || q >= nt + 1) {  // P, P', M and S chunks carry the tile record
-            r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
-            r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
-            r.V = V; r.all_coloc = md.all_coloc;
-            r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
-            r.P[0] = s_prod_pow[0]; r.P[1] = s_prod_pow[1]; r.P[2] = s_prod_pow[2];
-          } else if (q <= nt) {
-            for (int j = 0; j < kPairChunkViews && kPairChunkViews * (q - 1) + j < V; ++j) {
-              const View& w = s_prod_views[kPairChunkViews * (q - 1) + j];
-              r.cxy[j] = make_float4(w.cx, w.cx, w.cy, w.cy);
-              r.czz[j] = make_float4(w.cz, w.cz, 0.f, 0.f);
-              r.view[j] = w;
-            }
+        const MatDesc& md = s_prod_md;
+        const int T = md.H * md.W, V = md.V;
+        const int first = sq.z;
+        // the tile ends where the next one of its material starts
+        const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
+        const uint32_t bytes = (uint32_t)count * 4u;
+        const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
+        for (int q = 0; q < nt + 4; ++q) {
+          if (issued >= R) {
+            ok = __all_sync(0xffffffffu, wait_phase(smem_u32(&empty_bar[slot]), phase ^ 1u, err, kDevTimeoutEmpty));
+            if (!ok) break;
           }
-          mbar_arrive_expect_tx(fb, (uint32_t)nplanes * bytes);
+          const float* base;
+          int plane0, nplanes;
+          if (q == 0 || q == nt + 1) { base = md.tex; plane0 = 0; nplanes = 9; }
+          else if (q <= nt) {
+            base = md.tgt;
+            plane0 = 3 * kPairChunkViews * (q - 1);
+            nplanes = min(3 * kPairChunkViews, 3 * V - plane0);
+          }
+          else if (q == nt + 2) { base = md.m1; plane0 = 0; nplanes = 9; }
+          else { base = md.m2; plane0 = 0; nplanes = 9; }
+          const uint32_t fb = smem_u32(&full_bar[slot]);
+          if (lane == 0) {
+            PairSlotRec& r = recs[slot];
+            if (q == 0 || q >= nt + 1) {  // P, P', M and S chunks carry the tile record
+              r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
+              r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
+              r.V = V; r.all_coloc = md.all_coloc; r.count = count;
+              r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
+              r.P[0] = s_prod_pow[0]; r.P[1] = s_prod_pow[1]; r.P[2] = s_prod_pow[2];
+            } else if (q <= nt) {
+              for (int j = 0; j < kPairChunkViews && kPairChunkViews * (q - 1) + j < V; ++j) {
+                const View& w = s_prod_views[kPairChunkViews * (q - 1) + j];
+                r.cxy[j] = make_float4(w.cx, w.cx, w.cy, w.cy);
+                r.czz[j] = make_float4(w.cz, w.cz, 0.f, 0.f);
+                r.view[j] = w;
+              }
+            }
+            mbar_arrive_expect_tx(fb, (uint32_t)nplanes * bytes);
+          }
+          __syncwarp();
+          if (lane < nplanes)
+            bulk_g2s(ring_base + (uint32_t)(slot * SLOT + lane * TT) * 4u, base + (size_t)(plane0 + lane) * T + first,
+                     bytes, fb);
+          ++issued;
+          if (++slot == R) { slot = 0; phase ^= 1u; }
         }
-        __syncwarp();
-        if (lane < nplanes)
-          bulk_g2s(ring_base + (uint32_t)(slot * SLOT + lane * TT) * 4u, base + (size_t)(plane0 + lane) * T + first,
-                   bytes, fb);
-        ++issued;
-        if (++slot == R) { slot = 0; phase ^= 1u; }
       }
-    }
-    if (!ok && lane == 0) {
-      // drain: wait for the copies of the last min(R, issued) chunks to land
-      const long long n = issued < R ? issued : R;
-      int s = slot;
-      uint32_t ph = phase;
-      for (long long i = 0; i < n; ++i) {
-        if (--s < 0) { s = R - 1; ph ^= 1u; }
-        uint32_t it = 0;
-        while (!mbar_try_wait(smem_u32(&full_bar[s]), ph)) {
-          if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
+      if (!ok && was_ok && lane == 0) {
+        // drain: wait for the copies of the last min(R, issued) chunks to land
+        const long long n = issued < R ? issued : R;
+        int s = slot;
+        uint32_t ph = phase;
+        for (long long i = 0; i < n; ++i) {
+          if (--s < 0) { s = R - 1; ph ^= 1u; }
+          uint32_t it = 0;
+          while (!mbar_try_wait(smem_u32(&full_bar[s]), ph)) {
+            if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
+          }
         }
       }
-    }
-    __syncwarp();
-  } else {
-    // ------------------------------------------------------------ consumers
-    // A warp whose wait gave up (the error word is set) stops: no barrier among the
-    // consumer warps depends on it, and the launch's results are marked invalid.
-    const int tid = threadIdx.x;
-    RingCursor rc{0, 0u, true};
-    for (int k = k0; k < k1; ++k) {
-      const float2* pp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-      if (!rc.ok) break;
-      const PairSlotRec& r0 = recs[rc.slot];
-      const int first = r0.first, W = r0.W, V = r0.V;
-      const int T = W * r0.H;
-      // T is a multiple of 4 and tiles start at multiples of TT: both texels of a pair
-      // are in range or neither is
-      const bool active = 2 * tid < T - first;
-      const int idx = first + 2 * tid;
-      float2 px = make_float2(0.f, 0.f), py = make_float2(0.f, 0.f);
-      if (active) {
-        int i = (int)((float)idx * r0.inv_w);
-        int j = idx - i * W;
-        if (j < 0) { --i; j += W; }
-        else if (j >= W) { ++i; j -= W; }
-        int i1 = i, j1 = j + 1;
-        if (j1 == W) { j1 = 0; ++i1; }
-        // the planner's coordinate table, recomputed with the same IEEE operations
-        const float size = r0.size, fw = (float)W, fh = (float)r0.H;
-        px = make_float2(pixel_centre(j, fw, size), pixel_centre(j1, fw, size));
-        const float yi = -pixel_centre(i, fh, size);
-        py = make_float2(yi, i1 == i ? yi : -pixel_centre(i1, fh, size));
-      }
-      float2 g[9];
-      float2 pv[9];  // raw parameters of the second P copy
-      float2 loss2;
-      float2 gpl[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // dL/d light
-      bool live = true;
-      if (!GEN || r0.all_coloc) {
-        TexelPair u;
-        {
-          const float P[3] = {r0.P[0], r0.P[1], r0.P[2]};
+      __syncwarp();
+    } else {
+      // ------------------------------------------------------------ consumers
+      // A warp whose wait gave up (the error word is set) stops: no barrier among the
+      // consumer warps depends on it, and the launch's results are marked invalid.
+      const int tid = threadIdx.x;
+      for (int k = k0; k < k1; ++k) {
+        const float2* pp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+        if (!rc.ok) break;
+        const PairSlotRec& r0 = recs[rc.slot];
+        const int first = r0.first, W = r0.W, V = r0.V;
+        const int T = W * r0.H;
+        // T is a multiple of 4 and tiles start at multiples of 64: both texels of a pair are
+        // in range or neither is
+        const bool active = 2 * tid < r0.count;
+        if (64 * warp >= r0.count) {
+          // no texel of this tile belongs to this warp: it only lets the tile's slots pass
+          const int tile = r0.tile, chunks = (V + kPairChunkViews - 1) / kPairChunkViews + 4;
+          ring_release(rc, empty_bar, R);
+          for (int q = 1; q < chunks; ++q) {
+            pair_acquire<SLOT>(rc, ring, full_bar, err);
+            if (!rc.ok) break;
+            ring_release(rc, empty_bar, R);
+          }
+          if (!rc.ok) break;
+          if (lane == 0) warp_loss[(size_t)tile * NCW + warp] = 0.f;
+          if (lpart) write_light_partial(lpart, tile, NCW, 0.f, 0.f, 0.f);
+          continue;
+        }
+        const int idx = first + 2 * tid;
+        float2 px = make_float2(0.f, 0.f), py = make_float2(0.f, 0.f);
+        if (active) {
+          int i = (int)((float)idx * r0.inv_w);
+          int j = idx - i * W;
+          if (j < 0) { --i; j += W; }
+          else if (j >= W) { ++i; j -= W; }
+          int i1 = i, j1 = j + 1;
+          if (j1 == W) { j1 = 0; ++i1; }
+          // the planner's coordinate table, recomputed with the same IEEE operations
+          const float size = r0.size, fw = (float)W, fh = (float)r0.H;
+          px = make_float2(pixel_centre(j, fw, size), pixel_centre(j1, fw, size));
+          const float yi = -pixel_centre(i, fh, size);
+          py = make_float2(yi, i1 == i ? yi : -pixel_centre(i1, fh, size));
+        }
+        float2 g[9];
+        float2 pv[9];  // raw parameters of the second P copy
+        float2 loss2;
+        float2 gpl[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // dL/d light
+        bool live = true;
+        if (!GEN || r0.all_coloc) {
+          TexelPair u;
+          {
+            const float P[3] = {r0.P[0], r0.P[1], r0.P[2]};
+            float2 t9[9];
+#pragma unroll
+            for (int c = 0; c < 9; ++c) t9[c] = clamp2(pp[c * NT]);
+            ring_release(rc, empty_bar, R);
+            coloc_prepare_pair(t9, px, py, P, u);
+          }
+          AccC2 a;
+          acc2_zero(a);
+          for (int v0 = 0; v0 < V; v0 += kPairChunkViews) {
+            const float2* tp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+            if (!rc.ok) { live = false; break; }
+            const PairSlotRec& rv = recs[rc.slot];
+            const int nv = min(kPairChunkViews, V - v0);
+#pragma unroll
+            for (int j = 0; j < kPairChunkViews; ++j) {
+              if (j < nv) {
+                const float2 tg[3] = {tp[(3 * j) * NT], tp[(3 * j + 1) * NT], tp[(3 * j + 2) * NT]};
+                const float4 cxy = rv.cxy[j];
+                const float4 czz = rv.czz[j];
+                coloc_view_pair<LOSS>(u, make_float2(cxy.x, cxy.y), make_float2(cxy.z, cxy.w),
+                                      make_float2(czz.x, czz.y), tg, a);
+              }
+            }
+            ring_release(rc, empty_bar, R);
+          }
+          if (!live) break;
+          const float2* pq = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+          if (!rc.ok) break;
+          const PairSlotRec& r1 = recs[rc.slot];
+          const float P[3] = {r1.P[0], r1.P[1], r1.P[2]};
+          const float scale = r1.scale;
+#pragma unroll
+          for (int c = 0; c < 9; ++c) pv[c] = pq[c * NT];
+          ring_release(rc, empty_bar, R);
           float2 t9[9];
 #pragma unroll
-          for (int c = 0; c < 9; ++c) t9[c] = clamp2(pp[c * NT]);
-          ring_release(rc, empty_bar, R);
-          coloc_prepare_pair(t9, px, py, P, u);
-        }
-        AccC2 a;
-        acc2_zero(a);
-        for (int v0 = 0; v0 < V; v0 += kPairChunkViews) {
-          const float2* tp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-          if (!rc.ok) { live = false; break; }
-          const PairSlotRec& rv = recs[rc.slot];
-          const int nv = min(kPairChunkViews, V - v0);
+          for (int c = 0; c < 9; ++c) t9[c] = clamp2(pv[c]);
+          loss2 = coloc_finish_pair<LOSS>(t9, u, a, P, scale, g);
+          if (lpart) coloc_light_grad_pair<LOSS>(t9, a, scale, gpl);
+        } else {
+          // general views: the two texels one after the other through each chunk
+          const float P[3] = {r0.P[0], r0.P[1], r0.P[2]};
+          Maps ma, mb;
+          Adj aa, ab;
+          {
+            float ta[9], tb[9];
 #pragma unroll
-          for (int j = 0; j < kPairChunkViews; ++j) {
-            if (j < nv) {
-              const float2 tg[3] = {tp[(3 * j) * NT], tp[(3 * j + 1) * NT], tp[(3 * j + 2) * NT]};
-              const float4 cxy = rv.cxy[j];
-              const float4 czz = rv.czz[j];
-              coloc_view_pair<LOSS>(u, make_float2(cxy.x, cxy.y), make_float2(cxy.z, cxy.w),
-                                    make_float2(czz.x, czz.y), tg, a);
+            for (int c = 0; c < 9; ++c) {
+              const float2 t = clamp2(pp[c * NT]);
+              ta[c] = t.x;
+              tb[c] = t.y;
             }
+            ring_release(rc, empty_bar, R);
+            decode(ta, ma);
+            decode(tb, mb);
           }
+          adj_zero(aa);
+          adj_zero(ab);
+          float la = 0.f, lb = 0.f;
+          for (int v0 = 0; v0 < V; v0 += kPairChunkViews) {
+            const float2* tp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+            if (!rc.ok) { live = false; break; }
+            const PairSlotRec& rv = recs[rc.slot];
+            const int nv = min(kPairChunkViews, V - v0);
+            for (int j = 0; j < nv; ++j) {
+              const float2 t0 = tp[(3 * j) * NT], t1 = tp[(3 * j + 1) * NT], t2 = tp[(3 * j + 2) * NT];
+              const View& w = rv.view[j];
+              float ia[3] = {t0.x, t1.x, t2.x}, ib[3] = {t0.y, t1.y, t2.y};
+              if (w.coloc != 0.f) {
+                texel_view<kModeFused, LOSS, true, true>(ma, px.x, py.x, w, P, ia, la, aa);
+                texel_view<kModeFused, LOSS, true, true>(mb, px.y, py.y, w, P, ib, lb, ab);
+              } else {
+                texel_view<kModeFused, LOSS, true, false>(ma, px.x, py.x, w, P, ia, la, aa);
+                texel_view<kModeFused, LOSS, true, false>(mb, px.y, py.y, w, P, ib, lb, ab);
+              }
+            }
+            ring_release(rc, empty_bar, R);
+          }
+          if (!live) break;
+          const float2* pq = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+          if (!rc.ok) break;
+          const float scale = recs[rc.slot].scale;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) gpl[c] = make_float2(aa.gp[c] * scale, ab.gp[c] * scale);
+#pragma unroll
+          for (int c = 0; c < 9; ++c) pv[c] = pq[c * NT];
           ring_release(rc, empty_bar, R);
-        }
-        if (!live) break;
-        const float2* pq = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-        if (!rc.ok) break;
-        const PairSlotRec& r1 = recs[rc.slot];
-        const float P[3] = {r1.P[0], r1.P[1], r1.P[2]};
-        const float scale = r1.scale;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) pv[c] = pq[c * NT];
-        ring_release(rc, empty_bar, R);
-        float2 t9[9];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) t9[c] = clamp2(pv[c]);
-        loss2 = coloc_finish_pair<LOSS>(t9, u, a, P, scale, g);
-        if (lpart) coloc_light_grad_pair<LOSS>(t9, a, scale, gpl);
-      } else {
-        // general views: the two texels one after the other through each chunk
-        const float P[3] = {r0.P[0], r0.P[1], r0.P[2]};
-        Maps ma, mb;
-        Adj aa, ab;
-        {
-          float ta[9], tb[9];
+          float ta[9], tb[9], ga[9], gb[9];
 #pragma unroll
           for (int c = 0; c < 9; ++c) {
-            const float2 t = clamp2(pp[c * NT]);
+            const float2 t = clamp2(pv[c]);
             ta[c] = t.x;
             tb[c] = t.y;
           }
-          ring_release(rc, empty_bar, R);
-          decode(ta, ma);
-          decode(tb, mb);
+          adj_to_params(ta, ma, aa, scale, ga);
+          adj_to_params(tb, mb, ab, scale, gb);
+#pragma unroll
+          for (int c = 0; c < 9; ++c) g[c] = make_float2(ga[c], gb[c]);
+          loss2 = make_float2(la, lb);
         }
-        adj_zero(aa);
-        adj_zero(ab);
-        float la = 0.f, lb = 0.f;
-        for (int v0 = 0; v0 < V; v0 += kPairChunkViews) {
-          const float2* tp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-          if (!rc.ok) { live = false; break; }
-          const PairSlotRec& rv = recs[rc.slot];
-          const int nv = min(kPairChunkViews, V - v0);
-          for (int j = 0; j < nv; ++j) {
-            const float2 t0 = tp[(3 * j) * NT], t1 = tp[(3 * j + 1) * NT], t2 = tp[(3 * j + 2) * NT];
-            const View& w = rv.view[j];
-            float ia[3] = {t0.x, t1.x, t2.x}, ib[3] = {t0.y, t1.y, t2.y};
-            if (w.coloc != 0.f) {
-              texel_view<kModeFused, LOSS, true, true>(ma, px.x, py.x, w, P, ia, la, aa);
-              texel_view<kModeFused, LOSS, true, true>(mb, px.y, py.y, w, P, ib, lb, ab);
-            } else {
-              texel_view<kModeFused, LOSS, true, false>(ma, px.x, py.x, w, P, ia, la, aa);
-              texel_view<kModeFused, LOSS, true, false>(mb, px.y, py.y, w, P, ib, lb, ab);
-            }
+        // ---- Adam moments, update, write back (the destination comes from the S record)
+        float2 m1[9], m2[9];
+        {
+          const float2* sp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+          if (!rc.ok) break;
+#pragma unroll
+          for (int c = 0; c < 9; ++c) m1[c] = sp[c * NT];
+          ring_release(rc, empty_bar, R);
+        }
+        const float2* sp2 = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
+        if (!rc.ok) break;
+        const PairSlotRec& r3 = recs[rc.slot];
+        float* tex = r3.tex + idx;
+        float* gm1 = r3.m1 + idx;
+        float* gm2 = r3.m2 + idx;
+        const int tile = r3.tile;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) m2[c] = sp2[c * NT];
+        ring_release(rc, empty_bar, R);
+        float loss = 0.f;
+        if (active) {
+          const AdamScalars ad = s_adam[it];
+#pragma unroll
+          for (int c = 0; c < 9; ++c) {
+            float2 p = pv[c];
+            // textures.clamp(-1, 1): no gradient outside the range (nor for NaN)
+            const float2 gc = make_float2(fabsf(p.x) <= 1.0f ? g[c].x : 0.0f, fabsf(p.y) <= 1.0f ? g[c].y : 0.0f);
+            adam_update2(p, m1[c], m2[c], gc, ad);
+            const size_t off = (size_t)c * T;
+            *reinterpret_cast<float2*>(tex + off) = p;
+            *reinterpret_cast<float2*>(gm1 + off) = m1[c];
+            *reinterpret_cast<float2*>(gm2 + off) = m2[c];
           }
-          ring_release(rc, empty_bar, R);
+          loss = loss2.x + loss2.y;
         }
-        if (!live) break;
-        const float2* pq = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-        if (!rc.ok) break;
-        const float scale = recs[rc.slot].scale;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) gpl[c] = make_float2(aa.gp[c] * scale, ab.gp[c] * scale);
-#pragma unroll
-        for (int c = 0; c < 9; ++c) pv[c] = pq[c * NT];
-        ring_release(rc, empty_bar, R);
-        float ta[9], tb[9], ga[9], gb[9];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-          const float2 t = clamp2(pv[c]);
-          ta[c] = t.x;
-          tb[c] = t.y;
-        }
-        adj_to_params(ta, ma, aa, scale, ga);
-        adj_to_params(tb, mb, ab, scale, gb);
-#pragma unroll
-        for (int c = 0; c < 9; ++c) g[c] = make_float2(ga[c], gb[c]);
-        loss2 = make_float2(la, lb);
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (lane == 0) warp_loss[(size_t)tile * NCW + warp] = loss;
+        if (lpart)
+          write_light_partial(lpart, tile, NCW, active ? gpl[0].x + gpl[0].y : 0.f, active ? gpl[1].x + gpl[1].y : 0.f,
+                              active ? gpl[2].x + gpl[2].y : 0.f);
       }
-      // ---- Adam moments, update, write back (the destination comes from the S record)
-      float2 m1[9], m2[9];
-      {
-        const float2* sp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-        if (!rc.ok) break;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) m1[c] = sp[c * NT];
-        ring_release(rc, empty_bar, R);
-      }
-      const float2* sp2 = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
-      if (!rc.ok) break;
-      const PairSlotRec& r3 = recs[rc.slot];
-      float* tex = r3.tex + idx;
-      float* gm1 = r3.m1 + idx;
-      float* gm2 = r3.m2 + idx;
-      const int tile = r3.tile;
-#pragma unroll
-      for (int c = 0; c < 9; ++c) m2[c] = sp2[c * NT];
-      ring_release(rc, empty_bar, R);
-      float loss = 0.f;
-      if (active) {
-        const AdamScalars ad = s_adam;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-          float2 p = pv[c];
-          // textures.clamp(-1, 1): no gradient outside the range (nor for NaN)
-          const float2 gc = make_float2(fabsf(p.x) <= 1.0f ? g[c].x : 0.0f, fabsf(p.y) <= 1.0f ? g[c].y : 0.0f);
-          adam_update2(p, m1[c], m2[c], gc, ad);
-          const size_t off = (size_t)c * T;
-          *reinterpret_cast<float2*>(tex + off) = p;
-          *reinterpret_cast<float2*>(gm1 + off) = m1[c];
-          *reinterpret_cast<float2*>(gm2 + off) = m2[c];
-        }
-        loss = loss2.x + loss2.y;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-      if (lane == 0) warp_loss[(size_t)tile * NCW + warp] = loss;
-      if (lpart)
-        write_light_partial(lpart, tile, NCW, active ? gpl[0].x + gpl[0].y : 0.f, active ? gpl[1].x + gpl[1].y : 0.f,
-                            active ? gpl[2].x + gpl[2].y : 0.f);
     }
+    const bool more = it + 1 < iters;
+    // the maps and moments just stored are read by the next iteration's bulk copies
+    if (more) asm volatile("fence.proxy.async;" ::: "memory");
+    const bool last = batched_finish<NT + 32>(plan, hdr, mats, warp_loss, NCW, loss_hist, hist_len, step0 + 1 + it,
+                                              step_counter, ws + kWsCounter, &s_last, NCW, 1, lpart, &s_adam[it]);
+    if (more && !batched_next_iteration(last, ws, number0 + 1 + it, &s_last)) break;
+    if (more) asm volatile("fence.proxy.async;" ::: "memory");
   }
-  batched_finish<NT + 32>(plan, hdr, mats, warp_loss, NCW, loss_hist, hist_len, s_step, step_counter,
-                          ws + kWsCounter, &s_last, NCW, 1, lpart, &s_adam);
 }
 
 // ============================================================== variant 3: resident state
@@ -1159,7 +1240,7 @@ struct __align__(16) FuseStateRec {
   float* m2;
   float* unused;
   int tile, first, W, H;
-  int V, all_coloc, pad0, pad1;
+  int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
   float P[4];
 };
@@ -1229,7 +1310,9 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     fence_mbar_init();
     s_step = step0 + iters;
   }
-  for (int i = threadIdx.x; i < iters; i += blockDim.x) s_adam[i] = device_adam(hyper, step0 + 1 + i);
+  static_assert(kFuseMax <= 32, "one lane per iteration");
+  if (warp == 1 && lane < iters) adam_first(hyper, step0 + 1 + lane, s_adam[lane]);
+  if (warp == 2 && lane < iters) adam_second(hyper, step0 + 1 + lane, s_adam[lane]);
   __syncthreads();
   const int k0 = cta_off[blockIdx.x], k1 = cta_off[blockIdx.x + 1];
 
@@ -1246,7 +1329,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     int cur = -1;
     for (int k = k0; k < k1 && ok; ++k) {
       const int4 sq = sq_next;
-      if (k + 1 < k1) sq_next = seq[k + 1];
+      if (k + 1 < n_tiles) sq_next = seq[k + 1];
       if (sq.y != cur) {
         cur = sq.y;
         __syncwarp();
@@ -1259,7 +1342,9 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       const MatDesc& md = s_prod_md;
       const int T = md.H * md.W, V = md.V;
       const int first = sq.z;
-      const uint32_t bytes = (uint32_t)min(TT, T - first) * 4u;
+      // the tile ends where the next one of its material starts
+      const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
+      const uint32_t bytes = (uint32_t)count * 4u;
       const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
       // the state area is free once every consumer warp is done with the previous tile
       if (k > k0) {
@@ -1271,7 +1356,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         FuseStateRec& r = s_rec;
         r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
         r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
-        r.V = V; r.all_coloc = md.all_coloc;
+        r.V = V; r.all_coloc = md.all_coloc; r.count = count;
         r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
         r.P[0] = s_prod_pow[0]; r.P[1] = s_prod_pow[1]; r.P[2] = s_prod_pow[2];
         mbar_arrive_expect_tx(sfull, (uint32_t)kStatePlanes * bytes);
@@ -1346,12 +1431,25 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       const FuseStateRec& r0 = s_rec;
       const int V = r0.V;
       const bool coloc = !GEN || r0.all_coloc;
-      const bool active = 2 * tid < r0.W * r0.H - r0.first;
+      const bool active = 2 * tid < r0.count;
       bool live = true;
       // the pair's pixel centres, once per tile (they do not change across its iterations)
       float2 px = make_float2(0.f, 0.f), py = make_float2(0.f, 0.f);
       if (active) pair_coords(r0, tid, px, py);
-      for (int it = 0; it < iters; ++it) {
+      // a warp with no texel of this tile only lets the chunks pass, so that a tile smaller than
+      // the state area costs the warps it fills
+      const int chunks = (V + kPairChunkViews - 1) / kPairChunkViews;
+      const bool idle = 64 * warp >= r0.count;
+      for (int it = 0; idle && live && it < iters; ++it) {
+        for (int q = 0; q < chunks; ++q) {
+          pair_acquire<SLOT>(rc, ring, full_bar, err);
+          if (!rc.ok) { live = false; break; }
+          ring_release(rc, empty_bar, R);
+        }
+        if (lane == 0) warp_loss[((size_t)it * n_tiles + r0.tile) * NCW + warp] = 0.f;
+        if (lpart) write_light_partial(lpart, r0.tile, NCW, 0.f, 0.f, 0.f);
+      }
+      for (int it = 0; !idle && it < iters; ++it) {
         float2 g[9];
         float2 loss2;
         float2 gpl[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // dL/d light
@@ -1371,9 +1469,18 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
             if (!rc.ok) { live = false; break; }
             const PairSlotRec& rv = recs[rc.slot];
             const int nv = min(kPairChunkViews, V - v0);
+            if (nv == kPairChunkViews) {
 #pragma unroll
-            for (int j = 0; j < kPairChunkViews; ++j) {
-              if (j < nv) {
+              for (int j = 0; j < kPairChunkViews; ++j) {
+                const float2 tg[3] = {tp[(3 * j) * NT], tp[(3 * j + 1) * NT], tp[(3 * j + 2) * NT]};
+                const float4 cxy = rv.cxy[j];
+                const float4 czz = rv.czz[j];
+                coloc_view_pair<LOSS>(u, make_float2(cxy.x, cxy.y), make_float2(cxy.z, cxy.w),
+                                      make_float2(czz.x, czz.y), tg, a);
+              }
+            } else {
+#pragma unroll 1
+              for (int j = 0; j < nv; ++j) {
                 const float2 tg[3] = {tp[(3 * j) * NT], tp[(3 * j + 1) * NT], tp[(3 * j + 2) * NT]};
                 const float4 cxy = rv.cxy[j];
                 const float4 czz = rv.czz[j];
@@ -1870,10 +1977,16 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(unsigned* ws, uint32_
 // ============================================================== planner
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// One tile: `count` texels of material `mat` from texel `first`, run by CTA `cta`.
+struct TileRec {
+  int mat, first, count, cta;
+};
+
 struct PlanLayout {
   size_t off_mats, off_views, off_cta, off_order, off_tiles, off_mat_tiles, off_coords, off_seq, total;
   int n_tiles, n_ctas, total_views, ring;
   long long coord_floats;
+  std::vector<TileRec> tiles;  // variants 2 and 3
 };
 
 int resident_ctas(int variant, int threads);
@@ -1891,6 +2004,44 @@ static int fuse_ring(int threads, int variant) {
   const size_t state = fuse_state_bytes(threads);
   if (state >= budget) return 0;
   return (int)std::min<size_t>(kMaxRing, (budget - state) / pair_slot_bytes(threads));
+}
+
+// Cost of one texel of a V-view material, in views: the per-texel work besides the views
+// (set-up, map-back, Adam, parameter and moment traffic) is about 5 views.
+static double texel_cost(int views) { return views + 5.0; }
+
+// Tiles of the texel-pair variants (2 and 3). The materials' texels, in order, are dealt to the
+// CTAs in contiguous shares of equal cost, cut at multiples of a warp's 64 texels, and each
+// CTA's run of a material is divided into the fewest equal tiles of at most tile_texels. Tiles of
+// a fixed size instead leave a CTA up to one tile above the mean, which is most of the work
+// when a CTA has few of them: 512^2 texels are 273 tiles of 960 for 152 CTAs, two rounds of
+// which the second is 80 % full, and 256^2 are 69 tiles that leave half of the SMs without work.
+static void share_tiles(const svbrdf_material* mats, int n, int tile_texels, int ctas, std::vector<TileRec>& out) {
+  constexpr long long kGranule = 64;  // texels of one warp; keeps every tile's start 16-byte aligned
+  double total = 0.0;
+  for (int i = 0; i < n; ++i) total += (double)mats[i].height * mats[i].width * texel_cost(mats[i].n_views);
+  const double share = total / ctas;
+  double done = 0.0;  // cost dealt so far
+  int c = 0;
+  for (int i = 0; i < n; ++i) {
+    const long long T = (long long)mats[i].height * mats[i].width;
+    const double per = texel_cost(mats[i].n_views);
+    for (long long pos = 0; pos < T;) {
+      long long take = T - pos;
+      if (c < ctas - 1) {
+        const double room = ((c + 1) * share - done) / per;
+        const long long fit = (long long)(room / kGranule + 0.5) * kGranule;
+        if (fit <= 0) { ++c; continue; }
+        take = std::min(take, fit);
+      }
+      const long long k = (take + tile_texels - 1) / tile_texels;
+      const long long step = ((take + k - 1) / k + kGranule - 1) / kGranule * kGranule;
+      for (long long x = 0; x < take; x += step)
+        out.push_back(TileRec{i, (int)(pos + x), (int)std::min(step, take - x), c});
+      pos += take;
+      done += (double)take * per;
+    }
+  }
 }
 
 static int plan_layout(const svbrdf_material* mats, int n, const svbrdf_batch_config* cfg, PlanLayout& L) {
@@ -1954,7 +2105,15 @@ static int plan_layout(const svbrdf_material* mats, int n, const svbrdf_batch_co
   if (tiles > (1LL << 30)) return fail(SVBRDF_ERR_UNSUPPORTED, "too many tiles");
   int ctas = cfg->ctas > 0 ? cfg->ctas : resident_ctas(variant, cfg->threads);
   if (ctas <= 0) return fail(SVBRDF_ERR_CUDA, "could not query the device");
-  if (ctas > tiles) ctas = (int)tiles;
+  if (variant == 2 || variant == 3) {
+    long long granules = 0;
+    for (int i = 0; i < n; ++i) granules += ((long long)mats[i].height * mats[i].width + 63) / 64;
+    if (ctas > granules) ctas = (int)granules;
+    share_tiles(mats, n, cfg->tile_texels, ctas, L.tiles);
+    tiles = (long long)L.tiles.size();
+  } else {
+    if (ctas > tiles) ctas = (int)tiles;
+  }
   L.n_tiles = (int)tiles;
   L.n_ctas = ctas;
   L.total_views = views;
@@ -2228,6 +2387,46 @@ static size_t ws_slots(const PlanHeader* h) {
   return (size_t)h->n_tiles * (h->variant >= 1 ? (size_t)(h->threads / 32) : 1);
 }
 static size_t ws_loss_floats(const PlanHeader* h) { return ws_slots(h) * (h->variant >= 3 ? (size_t)kFuseMax : 1); }
+
+// The texel-pair kernel: a cooperative launch of `iters` iterations, or one of a single iteration
+// where the device cannot hold the whole grid at once (a grid set by the caller, fewer SMs for
+// this process) and where iters is 1.
+template <int LOSS, int NCW, bool GEN>
+static int launch_pair(const PlanHeader* h, const char* plan, int* step_counter, AdamHyper hyper, float* loss_hist,
+                       int hist_len, int& iters, unsigned* ws, float* part, float* lpart, cudaStream_t st) {
+  const int prc = pair_prepare<LOSS, NCW, GEN>(h->ring_slots);
+  if (prc) return prc;
+  const size_t smem = pair_smem<NCW>(h->ring_slots);
+  const auto kernel = batched_pair_kernel<LOSS, NCW, GEN>;
+  if (iters > 1) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (NCW + 1) * 32, smem) != cudaSuccess ||
+        (long long)per_sm * device_sm_count() < h->n_ctas) {
+      cudaGetLastError();
+      iters = 1;
+    }
+  }
+  cudaLaunchAttribute coop;
+  coop.id = cudaLaunchAttributeCooperative;
+  coop.val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(h->n_ctas);
+  cfg.blockDim = dim3((NCW + 1) * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &coop;
+  cfg.numAttrs = iters > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, plan, hyper, step_counter, loss_hist, hist_len, iters, part, ws, lpart);
+  if (e == cudaErrorCooperativeLaunchTooLarge && iters > 1) {
+    cudaGetLastError();
+    iters = 1;
+    cfg.numAttrs = 0;
+    e = cudaLaunchKernelEx(&cfg, kernel, plan, hyper, step_counter, loss_hist, hist_len, iters, part, ws, lpart);
+  }
+  if (e != cudaSuccess) return fail(SVBRDF_ERR_CUDA, "batched_pair_kernel: %s", cudaGetErrorString(e));
+  return SVBRDF_OK;
+}
+
 }  // namespace svb
 
 extern "C" {
@@ -2314,31 +2513,39 @@ int svbrdf_batched_plan(const svbrdf_material* materials, int n_materials, const
     if (!allc) h->general = 1;
     voff += m.n_views;
     mat_tiles[i] = t;
-    for (long long x = 0; x < T; x += config->tile_texels) {
-      tiles[t] = make_int2(i, (int)x);
-      const long long cnt = std::min<long long>(config->tile_texels, T - x);
-      // cost model: per-texel fixed work (set-up, map-back, Adam, parameter and moment
-      // traffic) ~ 5 views
-      cost[t] = (double)cnt * (m.n_views + 5.0);
-      total += cost[t];
-      ++t;
+    if (L.tiles.empty()) {
+      for (long long x = 0; x < T; x += config->tile_texels) {
+        tiles[t] = make_int2(i, (int)x);
+        cost[t] = (double)std::min<long long>(config->tile_texels, T - x) * texel_cost(m.n_views);
+        total += cost[t];
+        ++t;
+      }
+    } else {
+      for (; t < L.n_tiles && L.tiles[t].mat == i; ++t) {
+        tiles[t] = make_int2(i, L.tiles[t].first);
+        total += L.tiles[t].count * texel_cost(m.n_views);
+      }
     }
   }
   mat_tiles[n_materials] = t;
   h->total_cost = total;
-  // Contiguous split: CTA c takes the run of tiles (in material order) whose cost midpoints
-  // fall in its share [c, c+1) * total / n_ctas. Every CTA's load is within one tile of the
-  // mean, and a CTA crosses few material boundaries, so its consumers rarely re-stage a
-  // material's views and its producer rarely reloads a material.
+  for (int k = 0; k < L.n_tiles; ++k) order[k] = k;
   int kk = 0;
-  double acc = 0.0;
-  for (int c = 0; c < L.n_ctas; ++c) {
-    cta_off[c] = kk;
-    const double target = total * (double)(c + 1) / (double)L.n_ctas;
-    while (kk < L.n_tiles && (c == L.n_ctas - 1 || acc + 0.5 * cost[kk] <= target)) {
-      acc += cost[kk];
-      order[kk] = kk;
-      ++kk;
+  if (L.tiles.empty()) {
+    // Contiguous split: CTA c takes the run of tiles (in material order) whose cost midpoints
+    // fall in its share [c, c+1) * total / n_ctas. Every CTA's load is within one tile of the
+    // mean, and a CTA crosses few material boundaries, so its consumers rarely re-stage a
+    // material's views and its producer rarely reloads a material.
+    double acc = 0.0;
+    for (int c = 0; c < L.n_ctas; ++c) {
+      cta_off[c] = kk;
+      const double target = total * (double)(c + 1) / (double)L.n_ctas;
+      while (kk < L.n_tiles && (c == L.n_ctas - 1 || acc + 0.5 * cost[kk] <= target)) acc += cost[kk++];
+    }
+  } else {
+    for (int c = 0; c < L.n_ctas; ++c) {
+      cta_off[c] = kk;
+      while (kk < L.n_tiles && L.tiles[kk].cta == c) ++kk;
     }
   }
   cta_off[L.n_ctas] = L.n_tiles;
@@ -2371,10 +2578,12 @@ int svbrdf_batched_step(const void* device_plan, const void* host_plan, int loss
                               hist_len, 1, workspace, workspace_bytes, stream);
 }
 
-// One launch of the single-iteration variants (0, 1, 2).
-static int batched_launch_one(const PlanHeader* h, const char* plan, int loss_kind, int* step_counter,
-                              AdamHyper hyper, float* loss_hist, int hist_len, unsigned* ws, float* part,
-                              float* lpart, cudaStream_t st);
+// One launch of variants 0, 1 and 2: of `iters` iterations if that is above 1, the grid fits the
+// device at once and the device takes cooperative launches (variant 2 alone), else of one. `iters`
+// becomes the number that the launch runs.
+static int batched_launch_some(const PlanHeader* h, const char* plan, int loss_kind, int* step_counter,
+                               AdamHyper hyper, float* loss_hist, int hist_len, int& iters, unsigned* ws, float* part,
+                               float* lpart, cudaStream_t st);
 
 int svbrdf_batched_steps(const void* device_plan, const void* host_plan, int loss_kind, int* step_counter, float lr,
                          float beta1, float beta2, float eps, float* loss_hist, int hist_len, int iters,
@@ -2400,10 +2609,12 @@ int svbrdf_batched_steps(const void* device_plan, const void* host_plan, int los
   cudaStream_t st = (cudaStream_t)stream;
   const char* plan = (const char*)device_plan;
   if (h->variant < 3) {
-    for (int i = 0; i < iters; ++i) {
+    for (int i = 0; i < iters;) {
+      int k = h->variant == 2 && h->light ? std::min(iters - i, kFuseMax) : 1;
       const int rc =
-          batched_launch_one(h, plan, loss_kind, step_counter, hyper, loss_hist, hist_len, ws, part, lpart, st);
+          batched_launch_some(h, plan, loss_kind, step_counter, hyper, loss_hist, hist_len, k, ws, part, lpart, st);
       if (rc) return rc;
+      i += k;
     }
     return SVBRDF_OK;
   }
@@ -2444,9 +2655,9 @@ int svbrdf_batched_steps(const void* device_plan, const void* host_plan, int los
   return SVBRDF_OK;
 }
 
-static int batched_launch_one(const PlanHeader* h, const char* plan, int loss_kind, int* step_counter,
-                              AdamHyper hyper, float* loss_hist, int hist_len, unsigned* ws, float* part,
-                              float* lpart, cudaStream_t st) {
+static int batched_launch_some(const PlanHeader* h, const char* plan, int loss_kind, int* step_counter,
+                               AdamHyper hyper, float* loss_hist, int hist_len, int& iters, unsigned* ws, float* part,
+                               float* lpart, cudaStream_t st) {
   if (h->variant == 0) {
 #define SVB_B(L, NT) \
   batched_step_kernel<L, NT><<<h->n_ctas, NT, 0, st>>>(plan, hyper, step_counter, loss_hist, hist_len, part, ws)
@@ -2466,13 +2677,8 @@ static int batched_launch_one(const PlanHeader* h, const char* plan, int loss_ki
   const int ring = h->ring_slots;
   if (ring < 2 || ring > kMaxRing) return fail(SVBRDF_ERR_INVALID, "bad ring depth %d", ring);
   if (h->variant == 2) {
-#define SVB_P(L, NCW, G)                                                                                     \
-  {                                                                                                          \
-    int prc = pair_prepare<L, NCW, G>(ring);                                                                 \
-    if (prc) return prc;                                                                                     \
-    batched_pair_kernel<L, NCW, G><<<h->n_ctas, (NCW + 1) * 32, pair_smem<NCW>(ring), st>>>(                 \
-        plan, hyper, step_counter, loss_hist, hist_len, part, ws, lpart);                                    \
-  }
+#define SVB_P(L, NCW, G) \
+  return launch_pair<L, NCW, G>(h, plan, step_counter, hyper, loss_hist, hist_len, iters, ws, part, lpart, st);
 #define SVB_PG(L, NCW)         \
   if (h->general) SVB_P(L, NCW, true) \
   else SVB_P(L, NCW, false)
@@ -2481,16 +2687,15 @@ static int batched_launch_one(const PlanHeader* h, const char* plan, int loss_ki
   else if (loss_kind == SVBRDF_LOSS_LOG1P) SVB_PG(1, NCW) \
   else SVB_PG(2, NCW)
     switch (h->threads) {
-      case 224: SVB_PL(7) break;
-      case 256: SVB_PL(8) break;
-      case 384: SVB_PL(12) break;
-      case 480: SVB_PL(15) break;
-      default: SVB_PL(19) break;
+      case 224: SVB_PL(7)
+      case 256: SVB_PL(8)
+      case 384: SVB_PL(12)
+      case 480: SVB_PL(15)
+      default: SVB_PL(19)
     }
 #undef SVB_PG
 #undef SVB_PL
 #undef SVB_P
-    return check_launch("batched_pair_kernel");
   }
 #define SVB_T(L, NCW)                                                                                        \
   {                                                                                                          \

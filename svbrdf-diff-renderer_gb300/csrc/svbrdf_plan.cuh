@@ -4,7 +4,8 @@
 //   PlanHeader | MatDesc[n_mat] | View[total views] | int cta_off[n_ctas+1]
 //   | int order[n_tiles] | int2 tiles[n_tiles] (material, first texel)
 //   | int mat_tile_off[n_mat+1] | float coord tables (per material: x[W], then y[H])
-//   | int4 seq[n_tiles] (order[k]'s tile, material and first texel, in CTA order)
+//   | int4 seq[n_tiles] (order[k]'s tile, material and first texel, in CTA order; a tile
+//     of variants 2 and 3 ends where its material's next one starts, the others have tile_texels texels)
 // Tiles of one material are contiguous in tile-index order (mat_tile_off), so each
 // material's loss is a fixed-order sum over a tile range. cta_off[c]..cta_off[c+1]
 // indexes `order`, the planner's balanced permutation of tile ids for CTA c.
@@ -61,11 +62,13 @@ struct AdamHyper {
   float lr, beta1, beta2, eps;
 };
 
-// Workspace of a batched launch: [0] completion counter, [1] error word, then from byte
+// Workspace of a batched launch: [0] completion counter, [1] error word, [2] number of the last
+// iteration that a cooperative launch has finished (it only ever counts up), then from byte
 // 256 the per-(tile, warp) partial losses, then (plans with a learnable light) the
 // per-(tile, warp) partial light-power gradients, 3 floats each.
 constexpr int kWsCounter = 0;
 constexpr int kWsError = 1;
+constexpr int kWsIteration = 2;
 constexpr size_t kWsLossOffset = 256;
 
 // Error codes written to the workspace error word by a kernel that gave up waiting.
@@ -74,6 +77,7 @@ enum DeviceError : int {
   kDevTimeoutFull = 1,   // a consumer waited too long for a bulk copy
   kDevTimeoutEmpty = 2,  // the producer waited too long for consumers to free a slot
   kDevTimeoutDrain = 3,  // in-flight copies did not land while shutting down
+  kDevTimeoutGrid = 4,   // a CTA waited too long for the others to finish an iteration
 };
 
 }  // namespace svb

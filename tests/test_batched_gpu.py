@@ -261,3 +261,63 @@ def test_batched_learnable_light_matches_reference(svb, golden, cuda, variant):
     assert rel_l2(b.light_pow(0), d["light_pow"]) <= 1e-6
     ref = d["loss"].tolist()
     assert max(abs(float(b.loss_hist[k, 0]) - ref[k]) / ref[k] for k in range(len(ref))) <= 1e-5
+
+
+@pytest.mark.parametrize("variant,threads", [(2, 480), (2, 224), (3, 480), (3, 224), (3, 256)])
+@pytest.mark.parametrize("light", [False, True])
+def test_uneven_tiles_equal_single(svb, cuda, variant, threads, light):
+    """Tiles that leave warps without texels: a material of one pair of pairs (2 x 2), sizes with a
+    remainder of 4 texels after whole warps (18 x 18, 50 x 50), and more than one tile per CTA,
+    against the single-material kernel, with and without the learnable light."""
+    from oracle import microfacet_ref as R
+    mats = []
+    for i, res in enumerate((2, 18, 50, 130)):
+        sc = svb.scenes.Scene(res=res, size=17.0, camera_pos=svb.scenes.grid_views()[:5], gt=None,
+                              light_pos=svb.scenes.grid_views()[:5], light_pow=torch.full((3,), 1400.0), seed=i)
+        sc.gt = torch.rand(1, 9, res, res, generator=torch.Generator().manual_seed(i)) - 0.5
+        sc.init = svb.scenes.const_init(res)
+        svb.scenes.add_targets(sc, lambda *a: R.render(*a, dtype=torch.float32))
+        mats.append(sc)
+    b = svb.BatchedOptim(mats, lr=0.01, loss="mse", device=cuda, hist_len=6, optim_light=light,
+                         config=svb.BatchConfig(threads, 2 * threads, 9, variant))
+    b.run(6)
+    assert b.device_error() == 0
+    for i, m in enumerate(mats):
+        r = svb.Microfacet(m.res, m.n_views, m.size, [t.to(cuda) for t in m.cl], cuda)
+        o = svb.SvbrdfOptim(cuda, r, loss="mse", kernel="single")
+        o.load_targets(m.targets.to(cuda))
+        o.init_from_tex(m.init.to(cuda))
+        o.optim(6, 0.01, None, light)
+        assert rel_l2(b.tex[i], o.textures.detach()) <= 1e-6
+        assert rel_l2(b.m2[i], o.exp_avg_sq) <= 1e-5
+        for k in range(6):
+            assert abs(float(b.loss_hist[k, i]) - o.loss_image_list[k]) <= 1e-6 * o.loss_image_list[k]
+        if light:
+            assert rel_l2(b.light_pow(i), o.light_pow) <= 1e-6
+
+
+@pytest.mark.parametrize("threads,ctas,general", [(480, 0, False), (224, 0, False), (384, 7, True), (480, 1000, False)])
+def test_light_iterations_in_one_launch_match_single_steps(svb, cuda, threads, ctas, general):
+    """Variant 2 with the learnable light: 40 iterations as cooperative launches of 32 and 8, on the
+    whole device, on a few CTAs, and with a grid that the device cannot hold at once (which falls
+    back to one launch per iteration), give the same values as 40 single steps."""
+    mats = _batch(svb, cuda, n=4, general=general)
+    if ctas == 1000:
+        mats = [svb.scenes.single_scene(res=320, seed=3, device=cuda)]
+        mats[0].targets = torch.rand(9, 3, 320, 320, device=cuda)
+    runs = []
+    for many in (True, False):
+        b = svb.BatchedOptim(mats, device=cuda, config=svb.BatchConfig(threads, 2 * threads, ctas, 2), hist_len=40,
+                             optim_light=True)
+        if many:
+            b.run(40)
+        else:
+            for _ in range(40):
+                b.step()
+        assert b.device_error() == 0 and int(b.step_dev.item()) == 40
+        runs.append(b)
+    a, b = runs
+    assert torch.equal(a.loss_hist, b.loss_hist)
+    for i in range(len(mats)):
+        assert torch.equal(a.tex[i], b.tex[i]) and torch.equal(a.m2[i], b.m2[i])
+        assert torch.equal(a.light_pow(i), b.light_pow(i))

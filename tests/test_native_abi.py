@@ -345,3 +345,37 @@ def test_batched_render_loss_sums_and_conv_entries_reject_bad_arguments_on_host(
     # conv1_1's tensor-core data gradient: shape granularity and null pointers
     assert lib.svbrdf_desc_conv1_bwd_tc(fake, fake, fake, fake, 1, 12, 16, 1, err, None) == -2
     assert lib.svbrdf_desc_conv1_bwd_tc(fake, None, fake, fake, 1, 16, 16, 1, err, None) == -1
+
+
+@pytest.mark.parametrize("shapes", [[(256, 256, 9)], [(1024, 1024, 9)], [(2, 2, 3)], [(18, 18, 5)], [(512, 512, 16), (2, 2, 1)],
+                                    [(50, 50, 7), (130, 130, 3), (64, 66, 16)]])
+@pytest.mark.parametrize("threads,ctas,variant", [(480, 152, 3), (224, 304, 2), (384, 5, 3), (256, 1, 2)])
+def test_texel_pair_plan_shares(svb, lib, shapes, threads, ctas, variant):
+    """The texel-pair variants' tiles cover every texel once, start at multiples of a warp's 64
+    texels, fit the state area, and give every CTA the mean cost within one such step of texels
+    (a material's last texels, less than a step, go with the step before them)."""
+    SV = svb._native
+    mats, keep = _materials(SV, shapes)
+    cfg = SV.svbrdf_batch_config(threads, 2 * threads, ctas, variant)
+    nbytes = lib.svbrdf_batched_plan_bytes(mats, len(shapes), ctypes.byref(cfg))
+    buf = np.zeros(nbytes, np.uint8)
+    assert lib.svbrdf_batched_plan(mats, len(shapes), ctypes.byref(cfg), buf.ctypes.data, nbytes) == 0
+    hdr = np.frombuffer(buf[:72].tobytes(), np.int32)
+    n_tiles, n_ctas, off_cta, off_seq = hdr[2], hdr[3], hdr[8], hdr[16]
+    assert n_ctas == min(ctas, sum(-(-h * w // 64) for h, w, _ in shapes))
+    cta = np.frombuffer(buf[off_cta:off_cta + 4 * (n_ctas + 1)].tobytes(), np.int32)
+    seq = np.frombuffer(buf[off_seq:off_seq + 16 * n_tiles].tobytes(), np.int32).reshape(-1, 4)
+    assert cta[0] == 0 and cta[-1] == n_tiles and (np.diff(cta) >= 0).all()
+    counts, k = [], 0
+    for m, (h, w, _) in enumerate(shapes):
+        first = [int(s[2]) for s in seq if s[1] == m]
+        assert first[0] == 0 and all(f % 64 == 0 for f in first)
+        n = np.diff(first + [h * w])
+        assert (n > 0).all() and (n <= 2 * threads).all()
+        counts += n.tolist()
+        k += len(first)
+    assert k == n_tiles and seq[:, 0].tolist() == list(range(n_tiles))
+    cost = [c * (shapes[s[1]][2] + 5.0) for c, s in zip(counts, seq)]
+    loads = [sum(cost[cta[c]:cta[c + 1]]) for c in range(n_ctas)]
+    step = 64 * (max(v for _, _, v in shapes) + 5.0)
+    assert max(loads) <= sum(cost) / n_ctas + 1.5 * step
