@@ -248,24 +248,22 @@ __device__ __forceinline__ void texel_rc(int idx, const MatDesc& md, int& i, int
   else if (j >= md.W) { ++i; j -= md.W; }
 }
 
-// End of a batched launch, in every CTA: the warps' partial losses (`per_tile` per tile and
-// iteration; and with a learnable light, the light-gradient partials) of this CTA's own tiles
-// are summed per (iteration, tile) in warp order into the tile totals that follow the partials
-// in the workspace. The last CTA to finish then forms each material's mean loss from its
-// tiles' totals in tile order (a launch that ran `iters` iterations, steps step - iters + 1 ..
-// step, fills one loss_hist row per iteration), runs Adam on the learnable light powers, stores
-// the step counter and resets the completion counter. Both levels have a fixed order, so the
-// losses are deterministic; the last CTA reads one value per tile and iteration instead of
+// End of a launch of variants 0, 1 and 4, in every CTA: the warps' partial losses (`per_tile`
+// per tile and iteration) of this CTA's own tiles are summed per (iteration, tile) in warp
+// order into the tile totals that follow the partials in the workspace. The last CTA to finish
+// then forms each material's mean loss from its tiles' totals in tile order (a launch that ran
+// `iters` iterations, steps step - iters + 1 .. step, fills one loss_hist row per iteration),
+// stores the step counter and resets the completion counter. Both levels have a fixed order, so
+// the losses are deterministic; the last CTA reads one value per tile and iteration instead of
 // one per warp (15x fewer), in parallel across its warps.
 template <int NT>
-__device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeader* hdr, const MatDesc* mats,
+__device__ __forceinline__ void batched_finish(const char* plan, const PlanHeader* hdr, const MatDesc* mats,
                                                const float* partial, int per_tile, float* loss_hist, int hist_len,
                                                int step, int* step_counter, unsigned* counter, int* s_flag,
-                                               int nwarps, int iters = 1, const float* lpart = nullptr,
-                                               const AdamScalars* light_adam = nullptr) {
+                                               int nwarps, int iters = 1) {
   const int n_tiles = hdr->n_tiles;
   const size_t slots = (size_t)n_tiles * per_tile;
-  float* tile_tot = const_cast<float*>(partial) + slots * (hdr->variant >= 3 ? kFuseMax : 1) + (hdr->light ? 3 * slots : 0);
+  float* tile_tot = const_cast<float*>(partial) + slots * (hdr->variant >= 3 ? kFuseMax : 1);
   __syncthreads();  // every warp of this CTA has written its partials
   {
     const int* cta_off = (const int*)(plan + hdr->off_cta);
@@ -278,15 +276,6 @@ __device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeade
       for (int q = 0; q < per_tile; ++q) t += __ldcg(p + q);
       tile_tot[(size_t)i * n_tiles + tile] = t;
     }
-    if (lpart) {
-      for (int e = threadIdx.x; e < 3 * nk; e += blockDim.x) {
-        const int c = e / nk, tile = order[k0 + e % nk];
-        const float* p = lpart + 3 * (size_t)tile * per_tile + c;  // (tile, warp, channel)
-        float t = 0.f;
-        for (int q = 0; q < per_tile; ++q) t += __ldcg(p + 3 * q);
-        tile_tot[(size_t)(kFuseMax + c) * n_tiles + tile] = t;
-      }
-    }
     __threadfence();
   }
   __syncthreads();
@@ -296,7 +285,7 @@ __device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeade
     *s_flag = (prev == gridDim.x - 1) ? 1 : 0;
   }
   __syncthreads();
-  if (!*s_flag) return false;
+  if (!*s_flag) return;
   __threadfence();
   const int* mat_tiles = (const int*)(plan + hdr->off_mat_tiles);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -310,35 +299,115 @@ __device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeade
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) loss_hist[(size_t)((step - iters + i) % hist_len) * hdr->n_mat + mi] = (float)(acc * mats[mi].inv_n);
   }
-  if (lpart) {
-    // Learnable light (one-iteration launches): per material, the light-power gradient summed
-    // over its tiles in a fixed order, then Adam on the light with the maps' hyper-parameters
-    // and step (one optimiser over [textures, light_pow], src/svbrdf.py:50).
-    const AdamScalars ad = *light_adam;
-    for (int mi = w; mi < hdr->n_mat; mi += nw) {
-      const MatDesc& md = mats[mi];
-      if (!md.lstate) continue;
-      double g[3] = {0.0, 0.0, 0.0};
-      for (int t = mat_tiles[mi] + lane; t < mat_tiles[mi + 1]; t += 32) {
+  if (threadIdx.x == 0) {
+    *step_counter = step;
+    *counter = 0u;
+  }
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) g[c] += (double)__ldcg(tile_tot + (size_t)(kFuseMax + c) * n_tiles + t);
-      }
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Sums of the texel-pair kernels (variants 2 and 3). A CTA's tiles of one material in a row are a
+// run (the plan lists them). Each consumer warp adds its tiles' sums in tile order, in double, into
+// its own row of shared memory: row entry i is the loss of iteration i, or with a learnable light
+// (one iteration at a time) entry 0 is the loss and 1..3 the light-power gradient.
+struct RunSums {
+  double v[kFuseMax];
+};
+
+// The warp's sum of one tile and iteration: the lanes' values added in a fixed order.
+__device__ __forceinline__ void run_add(RunSums* row, int i, float v) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], o);
-      }
-      if (lane == 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          float p = md.lpow[c], m1 = md.lstate[c], m2 = md.lstate[3 + c];
-          adam_update(p, m1, m2, (float)g[c], ad);
-          md.lpow[c] = p;
-          md.lstate[c] = m1;
-          md.lstate[3 + c] = m2;
-        }
-      }
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) row->v[i] += (double)v;
+}
+
+// The run ends but the CTA goes on to another material: the warp's sums go to the workspace
+// (slot (run's first tile, warp); the light gradients to lpart) and start again at zero. The last
+// run's sums stay in shared memory for run_finish.
+__device__ __forceinline__ void run_flush(RunSums* row, int run_tile, int n_tiles, int ncw, int iters, float* partial,
+                                          float* lpart) {
+  __syncwarp();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t slot = (size_t)run_tile * ncw + warp;
+  if (lane < iters) partial[(size_t)lane * n_tiles * ncw + slot] = (float)row->v[lane];
+  if (lpart && lane >= 1 && lane <= 3) lpart[3 * slot + lane - 1] = (float)row->v[lane];
+  row->v[lane] = 0.0;
+  __syncwarp();
+}
+
+// End of a launch (or of an iteration of a cooperative one), in every CTA: the warps' sums of
+// each of the CTA's runs are added into one total per run and quantity; the last CTA to finish
+// adds each material's run totals in run order, fills the loss history, steps the learnable
+// lights and resets the completion counter. Every level has a fixed order, so losses and lights
+// are deterministic. A warp forms one total with one load per lane and a shuffle tree, and the
+// last CTA reads one value per (run, quantity), at most one per CTA of each material: the tile
+// totals that this replaces took a serial sum over the warps, and one value per tile, and with
+// one 512^2 material with a learnable light took 32.5 us per iteration where it now takes 27.
+template <int NCW>
+__device__ __forceinline__ bool run_finish(const char* plan, const PlanHeader* hdr, const MatDesc* mats,
+                                           const RunSums* rows, float* partial, float* lpart, float* loss_hist,
+                                           int hist_len, int step, int* step_counter, unsigned* counter, int* s_flag,
+                                           int iters, const AdamScalars* light_adam) {
+  const int n_tiles = hdr->n_tiles, nq = lpart ? 4 : iters;
+  const size_t slots = (size_t)n_tiles * NCW;
+  float* totals = partial + slots * (hdr->variant >= 3 ? kFuseMax : 1) + (hdr->light ? 3 * slots : 0);
+  const int* run_tile = (const int*)(plan + hdr->off_runs);
+  const int* cta_run = (const int*)(plan + hdr->off_cta_run);
+  const int* mat_run = (const int*)(plan + hdr->off_mat_run);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = cta_run[blockIdx.x], nr = cta_run[blockIdx.x + 1] - r0;
+  __syncthreads();  // every warp of this CTA is done with its tiles
+  for (int e = w; e < nr * nq; e += NCW + 1) {
+    const int r = e / nq, q = e % nq, tile = run_tile[r0 + r];
+    const size_t slot = (size_t)tile * NCW + lane;
+    double v = 0.0;
+    if (lane < NCW) {
+      if (r == nr - 1) v = rows[lane].v[q];
+      else if (lpart && q > 0) v = (double)__ldcg(lpart + 3 * slot + q - 1);
+      else v = (double)__ldcg(partial + (size_t)q * slots + slot);
     }
+    v = warp_sum(v);
+    if (lane == 0) {
+      totals[(size_t)(lpart && q > 0 ? kFuseMax + q - 1 : q) * n_tiles + tile] = (float)v;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *s_flag = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1 : 0;
+  }
+  __syncthreads();
+  if (!*s_flag) return false;
+  __threadfence();
+  // one warp per (material, quantity)
+  for (int e = w; e < hdr->n_mat * nq; e += NCW + 1) {
+    const int mi = e / nq, q = e % nq;
+    const MatDesc& md = mats[mi];
+    const bool light = lpart && q > 0;
+    if (light && !md.lstate) continue;
+    const float* tt = totals + (size_t)(light ? kFuseMax + q - 1 : q) * n_tiles;
+    double acc = 0.0;
+    for (int r = mat_run[mi] + lane; r < mat_run[mi + 1]; r += 32) acc += (double)__ldcg(tt + run_tile[r]);
+    acc = warp_sum(acc);
+    if (lane != 0) continue;
+    if (!light) {
+      loss_hist[(size_t)((step - iters + q) % hist_len) * hdr->n_mat + mi] = (float)(acc * md.inv_n);
+      continue;
+    }
+    // Adam on the light power with the maps' hyper-parameters and step (one optimiser over
+    // [textures, light_pow], src/svbrdf.py:50)
+    const int c = q - 1;
+    float p = __ldcg(md.lpow + c), m1 = __ldcg(md.lstate + c), m2 = __ldcg(md.lstate + 3 + c);
+    adam_update(p, m1, m2, (float)acc, *light_adam);
+    md.lpow[c] = p;
+    md.lstate[c] = m1;
+    md.lstate[3 + c] = m2;
   }
   if (threadIdx.x == 0) {
     *step_counter = step;
@@ -347,7 +416,7 @@ __device__ __forceinline__ bool batched_finish(const char* plan, const PlanHeade
   return true;
 }
 
-// End of an iteration inside a cooperative launch: the last CTA, whose writes in batched_finish
+// End of an iteration inside a cooperative launch: the last CTA, whose writes in run_finish
 // come first, publishes the iteration's number in ws[kWsIteration]; the others wait for it. The
 // wait is bounded (about a second of polls); false in every thread if it ran out.
 __device__ __forceinline__ bool batched_next_iteration(bool last, unsigned* ws, unsigned number, int* s_flag) {
@@ -374,23 +443,6 @@ __device__ __forceinline__ bool batched_next_iteration(bool last, unsigned* ws, 
   }
   __syncthreads();
   return *s_flag != 0;
-}
-
-// Light-power gradient partial of one warp's texels of one tile: lanes' values summed in a
-// fixed order, written by lane 0 to slot (tile, warp).
-__device__ __forceinline__ void write_light_partial(float* lpart, int tile, int nwarps, float s0, float s1, float s2) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    float* p = lpart + 3 * ((size_t)tile * nwarps + (threadIdx.x >> 5));
-    p[0] = s0;
-    p[1] = s1;
-    p[2] = s2;
-  }
 }
 
 // ============================================================== variant 0: direct loads
@@ -831,7 +883,7 @@ batched_tma_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restri
 // kFuseMax iterations run in one cooperative launch: at the end of each, the last CTA to arrive
 // reduces and steps the light (batched_finish) and the others wait for it. One launch per
 // iteration paid its start (launch, plan and Adam scalars, an empty ring) and its drain each
-// time: on one 512^2 material with 9 views 33 us per iteration; the cooperative form LIGHT_US us.
+// time, about 4 us of the 27 of one 512^2 material with 9 views.
 constexpr int kPairSlotPlanes = 9;
 constexpr int kPairChunkViews = 3;
 constexpr size_t kPairRingBudget = 216 * 1024;
@@ -865,7 +917,7 @@ struct __align__(16) PairSlotRec {
   float* tex;                   // P chunks: the tile's material ...
   float* m1;
   float* m2;
-  float* unused;
+  int run_tile, run_ends;       // the run's first tile; 1 if it ends here and another follows
   int tile, first, W, H;        // ... tile id and first texel
   int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
@@ -887,6 +939,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   __shared__ View s_prod_views[kMaxViews];  // ... its views
   __shared__ float s_prod_pow[4];           // ... and light power
   __shared__ AdamScalars s_adam[kFuseMax];
+  __shared__ RunSums s_sums[NCW];
   __shared__ int s_last;
 
   const PlanHeader* hdr = (const PlanHeader*)plan;
@@ -930,12 +983,13 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       const int4* seq = (const int4*)(plan + hdr->off_seq);
       const bool was_ok = ok;
       int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
-      int cur = -1;
+      int cur = -1, run_tile = 0;
       for (int k = k0; k < k1 && ok; ++k) {
         const int4 sq = sq_next;
         if (k + 1 < n_tiles) sq_next = seq[k + 1];
         if (sq.y != cur) {
           cur = sq.y;
+          run_tile = sq.x;
           __syncwarp();
           const MatDesc& m = mats[cur];
           if (lane == 0) s_prod_md = m;
@@ -949,6 +1003,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         // the tile ends where the next one of its material starts
         const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
         const uint32_t bytes = (uint32_t)count * 4u;
+        const int run_ends = k + 1 < k1 && sq_next.y != cur;
         const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
         for (int q = 0; q < nt + 4; ++q) {
           if (issued >= R) {
@@ -972,6 +1027,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
               r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
               r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
               r.V = V; r.all_coloc = md.all_coloc; r.count = count;
+              r.run_tile = run_tile; r.run_ends = run_ends;
               r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
               r.P[0] = s_prod_pow[0]; r.P[1] = s_prod_pow[1]; r.P[2] = s_prod_pow[2];
             } else if (q <= nt) {
@@ -1011,6 +1067,8 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       // A warp whose wait gave up (the error word is set) stops: no barrier among the
       // consumer warps depends on it, and the launch's results are marked invalid.
       const int tid = threadIdx.x;
+      s_sums[warp].v[lane] = 0.0;
+      __syncwarp();
       for (int k = k0; k < k1; ++k) {
         const float2* pp = pair_acquire<SLOT>(rc, ring, full_bar, err) + tid;
         if (!rc.ok) break;
@@ -1022,7 +1080,8 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         const bool active = 2 * tid < r0.count;
         if (64 * warp >= r0.count) {
           // no texel of this tile belongs to this warp: it only lets the tile's slots pass
-          const int tile = r0.tile, chunks = (V + kPairChunkViews - 1) / kPairChunkViews + 4;
+          const int chunks = (V + kPairChunkViews - 1) / kPairChunkViews + 4;
+          const int run_tile = r0.run_tile, run_ends = r0.run_ends;
           ring_release(rc, empty_bar, R);
           for (int q = 1; q < chunks; ++q) {
             pair_acquire<SLOT>(rc, ring, full_bar, err);
@@ -1030,8 +1089,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
             ring_release(rc, empty_bar, R);
           }
           if (!rc.ok) break;
-          if (lane == 0) warp_loss[(size_t)tile * NCW + warp] = 0.f;
-          if (lpart) write_light_partial(lpart, tile, NCW, 0.f, 0.f, 0.f);
+          if (run_ends) run_flush(&s_sums[warp], run_tile, n_tiles, NCW, 1, warp_loss, lpart);
           continue;
         }
         const int idx = first + 2 * tid;
@@ -1173,7 +1231,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         float* tex = r3.tex + idx;
         float* gm1 = r3.m1 + idx;
         float* gm2 = r3.m2 + idx;
-        const int tile = r3.tile;
+        const int run_tile = r3.run_tile, run_ends = r3.run_ends;
 #pragma unroll
         for (int c = 0; c < 9; ++c) m2[c] = sp2[c * NT];
         ring_release(rc, empty_bar, R);
@@ -1193,19 +1251,19 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
           }
           loss = loss2.x + loss2.y;
         }
+        run_add(&s_sums[warp], 0, loss);
+        if (lpart) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-        if (lane == 0) warp_loss[(size_t)tile * NCW + warp] = loss;
-        if (lpart)
-          write_light_partial(lpart, tile, NCW, active ? gpl[0].x + gpl[0].y : 0.f, active ? gpl[1].x + gpl[1].y : 0.f,
-                              active ? gpl[2].x + gpl[2].y : 0.f);
+          for (int c = 0; c < 3; ++c) run_add(&s_sums[warp], 1 + c, active ? gpl[c].x + gpl[c].y : 0.f);
+        }
+        if (run_ends) run_flush(&s_sums[warp], run_tile, n_tiles, NCW, 1, warp_loss, lpart);
       }
     }
     const bool more = it + 1 < iters;
     // the maps and moments just stored are read by the next iteration's bulk copies
     if (more) asm volatile("fence.proxy.async;" ::: "memory");
-    const bool last = batched_finish<NT + 32>(plan, hdr, mats, warp_loss, NCW, loss_hist, hist_len, step0 + 1 + it,
-                                              step_counter, ws + kWsCounter, &s_last, NCW, 1, lpart, &s_adam[it]);
+    const bool last = run_finish<NCW>(plan, hdr, mats, s_sums, warp_loss, lpart, loss_hist, hist_len, step0 + 1 + it,
+                                      step_counter, ws + kWsCounter, &s_last, 1, &s_adam[it]);
     if (more && !batched_next_iteration(last, ws, number0 + 1 + it, &s_last)) break;
     if (more) asm volatile("fence.proxy.async;" ::: "memory");
   }
@@ -1238,7 +1296,7 @@ struct __align__(16) FuseStateRec {
   float* tex;
   float* m1;
   float* m2;
-  float* unused;
+  int run_tile, run_ends;  // the run's first tile; 1 if it ends here and another follows
   int tile, first, W, H;
   int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
@@ -1286,7 +1344,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   __shared__ View s_prod_views[kMaxViews];
   __shared__ float s_prod_pow[4];
   __shared__ AdamScalars s_adam[kFuseMax];
-  __shared__ int s_step;
+  __shared__ RunSums s_sums[NCW];
   __shared__ int s_last;
 
   const PlanHeader* hdr = (const PlanHeader*)plan;
@@ -1308,7 +1366,6 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     mbar_init(smem_u32(&state_full), 1);
     mbar_init(smem_u32(&state_empty), NCW);
     fence_mbar_init();
-    s_step = step0 + iters;
   }
   static_assert(kFuseMax <= 32, "one lane per iteration");
   if (warp == 1 && lane < iters) adam_first(hyper, step0 + 1 + lane, s_adam[lane]);
@@ -1326,12 +1383,13 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     long long issued = 0, states = 0;
     bool ok = true;
     int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
-    int cur = -1;
+    int cur = -1, run_tile = 0;
     for (int k = k0; k < k1 && ok; ++k) {
       const int4 sq = sq_next;
       if (k + 1 < n_tiles) sq_next = seq[k + 1];
       if (sq.y != cur) {
         cur = sq.y;
+        run_tile = sq.x;
         __syncwarp();
         const MatDesc& m = mats[cur];
         if (lane == 0) s_prod_md = m;
@@ -1345,6 +1403,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       // the tile ends where the next one of its material starts
       const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
       const uint32_t bytes = (uint32_t)count * 4u;
+      const int run_ends = k + 1 < k1 && sq_next.y != cur;
       const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
       // the state area is free once every consumer warp is done with the previous tile
       if (k > k0) {
@@ -1357,6 +1416,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
         r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
         r.V = V; r.all_coloc = md.all_coloc; r.count = count;
+        r.run_tile = run_tile; r.run_ends = run_ends;
         r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
         r.P[0] = s_prod_pow[0]; r.P[1] = s_prod_pow[1]; r.P[2] = s_prod_pow[2];
         mbar_arrive_expect_tx(sfull, (uint32_t)kStatePlanes * bytes);
@@ -1422,6 +1482,8 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     const float2* sp = sw;
     RingCursor rc{0, 0u, true};
     uint32_t sfp = 0;
+    s_sums[warp].v[lane] = 0.0;
+    __syncwarp();
     for (int k = k0; k < k1; ++k) {
       if (rc.ok) rc.ok = __all_sync(0xffffffffu, wait_phase(smem_u32(&state_full), sfp, err, kDevTimeoutFull));
       sfp ^= 1u;
@@ -1446,8 +1508,6 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
           if (!rc.ok) { live = false; break; }
           ring_release(rc, empty_bar, R);
         }
-        if (lane == 0) warp_loss[((size_t)it * n_tiles + r0.tile) * NCW + warp] = 0.f;
-        if (lpart) write_light_partial(lpart, r0.tile, NCW, 0.f, 0.f, 0.f);
       }
       for (int it = 0; !idle && it < iters; ++it) {
         float2 g[9];
@@ -1579,22 +1639,22 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
           }
           loss = loss2.x + loss2.y;
         }
+        run_add(&s_sums[warp], it, loss);
+        if (lpart) {  // plans with a learnable light run one iteration per launch
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-        if (lane == 0) warp_loss[((size_t)it * n_tiles + r0.tile) * NCW + warp] = loss;
-        if (lpart)  // plans with a learnable light run one iteration per launch
-          write_light_partial(lpart, r0.tile, NCW, active ? gpl[0].x + gpl[0].y : 0.f,
-                              active ? gpl[1].x + gpl[1].y : 0.f, active ? gpl[2].x + gpl[2].y : 0.f);
+          for (int c = 0; c < 3; ++c) run_add(&s_sums[warp], 1 + c, active ? gpl[c].x + gpl[c].y : 0.f);
+        }
       }
       if (!live) break;
+      if (r0.run_ends) run_flush(&s_sums[warp], r0.run_tile, n_tiles, NCW, iters, warp_loss, lpart);
       // this warp's shared-memory writes come before the next tile's bulk copies into the area
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&state_empty));
     }
   }
-  batched_finish<NT + 32>(plan, hdr, mats, warp_loss, NCW, loss_hist, hist_len, s_step, step_counter,
-                          ws + kWsCounter, &s_last, NCW, iters, lpart, &s_adam[0]);
+  run_finish<NCW>(plan, hdr, mats, s_sums, warp_loss, lpart, loss_hist, hist_len, step0 + iters, step_counter,
+                  ws + kWsCounter, &s_last, iters, &s_adam[0]);
 }
 
 // ============================================================== variant 4: resident state, no producer
@@ -1983,8 +2043,8 @@ struct TileRec {
 };
 
 struct PlanLayout {
-  size_t off_mats, off_views, off_cta, off_order, off_tiles, off_mat_tiles, off_coords, off_seq, total;
-  int n_tiles, n_ctas, total_views, ring;
+  size_t off_mats, off_views, off_cta, off_order, off_tiles, off_mat_tiles, off_coords, off_seq, off_runs, off_cta_run, off_mat_run, total;
+  int n_tiles, n_ctas, n_runs, total_views, ring;
   long long coord_floats;
   std::vector<TileRec> tiles;  // variants 2 and 3
 };
@@ -2042,6 +2102,11 @@ static void share_tiles(const svbrdf_material* mats, int n, int tile_texels, int
       done += (double)take * per;
     }
   }
+}
+
+// Whether tile k starts a run: a CTA's consecutive tiles of one material.
+static bool run_starts(const std::vector<TileRec>& t, size_t k) {
+  return k == 0 || t[k].cta != t[k - 1].cta || t[k].mat != t[k - 1].mat;
 }
 
 static int plan_layout(const svbrdf_material* mats, int n, const svbrdf_batch_config* cfg, PlanLayout& L) {
@@ -2111,7 +2176,10 @@ static int plan_layout(const svbrdf_material* mats, int n, const svbrdf_batch_co
     if (ctas > granules) ctas = (int)granules;
     share_tiles(mats, n, cfg->tile_texels, ctas, L.tiles);
     tiles = (long long)L.tiles.size();
+    L.n_runs = 0;
+    for (size_t k = 0; k < L.tiles.size(); ++k) L.n_runs += run_starts(L.tiles, k);
   } else {
+    L.n_runs = 0;
     if (ctas > tiles) ctas = (int)tiles;
   }
   L.n_tiles = (int)tiles;
@@ -2139,6 +2207,9 @@ static int plan_layout(const svbrdf_material* mats, int n, const svbrdf_batch_co
   L.off_mat_tiles = o; o += sizeof(int) * (n + 1); o = align_up(o, 16);
   L.off_coords = o; o += sizeof(float) * coords; o = align_up(o, 16);
   L.off_seq = o; o += sizeof(int4) * tiles; o = align_up(o, 16);
+  L.off_runs = o; o += sizeof(int) * L.n_runs; o = align_up(o, 16);
+  L.off_cta_run = o; o += sizeof(int) * (ctas + 1); o = align_up(o, 16);
+  L.off_mat_run = o; o += sizeof(int) * (n + 1); o = align_up(o, 16);
   L.total = o;
   if (L.total > (size_t)0x7fffffff) return fail(SVBRDF_ERR_UNSUPPORTED, "plan too large");
   return SVBRDF_OK;
@@ -2461,6 +2532,9 @@ int svbrdf_batched_plan(const svbrdf_material* materials, int n_materials, const
   h->off_mat_tiles = (int)L.off_mat_tiles;
   h->off_coords = (int)L.off_coords;
   h->off_seq = (int)L.off_seq;
+  h->off_runs = (int)L.off_runs;
+  h->off_cta_run = (int)L.off_cta_run;
+  h->off_mat_run = (int)L.off_mat_run;
   h->variant = config->variant;
   h->ring_slots = L.ring;
   h->total_bytes = (long long)L.total;
@@ -2543,10 +2617,21 @@ int svbrdf_batched_plan(const svbrdf_material* materials, int n_materials, const
       while (kk < L.n_tiles && (c == L.n_ctas - 1 || acc + 0.5 * cost[kk] <= target)) acc += cost[kk++];
     }
   } else {
+    int* runs = (int*)(base + L.off_runs);
+    int* cta_run = (int*)(base + L.off_cta_run);
+    int* mat_run = (int*)(base + L.off_mat_run);
+    int r = 0, m = 0;
     for (int c = 0; c < L.n_ctas; ++c) {
       cta_off[c] = kk;
-      while (kk < L.n_tiles && L.tiles[kk].cta == c) ++kk;
+      cta_run[c] = r;
+      for (; kk < L.n_tiles && L.tiles[kk].cta == c; ++kk) {
+        if (!run_starts(L.tiles, kk)) continue;
+        while (m <= L.tiles[kk].mat) mat_run[m++] = r;
+        runs[r++] = kk;
+      }
     }
+    cta_run[L.n_ctas] = r;
+    while (m <= n_materials) mat_run[m++] = r;
   }
   cta_off[L.n_ctas] = L.n_tiles;
   int4* seq = (int4*)(base + L.off_seq);

@@ -6,6 +6,7 @@
 //   | int mat_tile_off[n_mat+1] | float coord tables (per material: x[W], then y[H])
 //   | int4 seq[n_tiles] (order[k]'s tile, material and first texel, in CTA order; a tile
 //     of variants 2 and 3 ends where its material's next one starts, the others have tile_texels texels)
+//   | variants 2 and 3: int run_tile[n_runs] | int cta_run[n_ctas+1] | int mat_run[n_mat+1]
 // Tiles of one material are contiguous in tile-index order (mat_tile_off), so each
 // material's loss is a fixed-order sum over a tile range. cta_off[c]..cta_off[c+1]
 // indexes `order`, the planner's balanced permutation of tile ids for CTA c.
@@ -34,6 +35,9 @@ struct PlanHeader {
   int general;      // 1 when some material has a view whose light is not at the camera
   int off_seq;      // int4 (tile, material, first texel, 0) per entry of `order`
   int light;        // 1 when some material's light power is learnable (MatDesc::lstate)
+  int off_runs;     // variants 2 and 3: first tile of each run (a CTA's tiles of one material) ...
+  int off_cta_run;  // ... the first run of each CTA [n_ctas + 1] ...
+  int off_mat_run;  // ... and of each material [n_mat + 1]
   long long total_bytes;
   double total_cost;
 };

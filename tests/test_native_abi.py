@@ -360,7 +360,7 @@ def test_texel_pair_plan_shares(svb, lib, shapes, threads, ctas, variant):
     nbytes = lib.svbrdf_batched_plan_bytes(mats, len(shapes), ctypes.byref(cfg))
     buf = np.zeros(nbytes, np.uint8)
     assert lib.svbrdf_batched_plan(mats, len(shapes), ctypes.byref(cfg), buf.ctypes.data, nbytes) == 0
-    hdr = np.frombuffer(buf[:72].tobytes(), np.int32)
+    hdr = np.frombuffer(buf[:84].tobytes(), np.int32)
     n_tiles, n_ctas, off_cta, off_seq = hdr[2], hdr[3], hdr[8], hdr[16]
     assert n_ctas == min(ctas, sum(-(-h * w // 64) for h, w, _ in shapes))
     cta = np.frombuffer(buf[off_cta:off_cta + 4 * (n_ctas + 1)].tobytes(), np.int32)
@@ -379,3 +379,11 @@ def test_texel_pair_plan_shares(svb, lib, shapes, threads, ctas, variant):
     loads = [sum(cost[cta[c]:cta[c + 1]]) for c in range(n_ctas)]
     step = 64 * (max(v for _, _, v in shapes) + 5.0)
     assert max(loads) <= sum(cost) / n_ctas + 1.5 * step
+    # runs: a CTA's consecutive tiles of one material, listed per CTA and per material
+    starts = sorted({int(cta[c]) for c in range(n_ctas) if cta[c] < cta[c + 1]} |
+                    {i for i in range(n_tiles) if i == 0 or seq[i][1] != seq[i - 1][1]})
+    ints = lambda off, n: np.frombuffer(buf[off:off + 4 * n].tobytes(), np.int32)
+    assert ints(hdr[18], len(starts)).tolist() == starts
+    cta_run, mat_run = ints(hdr[19], n_ctas + 1), ints(hdr[20], len(shapes) + 1)
+    assert [sum(s < cta[c] for s in starts) for c in range(n_ctas + 1)] == cta_run.tolist()
+    assert [sum(seq[s][1] < m for s in starts) for m in range(len(shapes) + 1)] == mat_run.tolist()
