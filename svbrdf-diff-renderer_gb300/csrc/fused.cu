@@ -1285,7 +1285,9 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
 // warp) partials, so the loss history equals K separate launches'. The state area is
 // single-buffered: the producer reloads it once every consumer warp has signalled it done
 // with the tile (state_empty), after a proxy fence orders their shared-memory writes before
-// the bulk copies. Waits, error recording and draining follow variant 2.
+// the bulk copies. Waits, error recording and draining follow variant 2. Plans with a learnable
+// light launch the GEN instantiation (one iteration at a time): without that code the co-located
+// one is 1 % faster.
 constexpr int kStatePlanes = 27;
 constexpr size_t kFuseBudget = 220 * 1024;
 constexpr size_t kFuseBudgetTwoCta = 100 * 1024;
@@ -1327,7 +1329,8 @@ template <int LOSS, int NCW, bool GEN>
 __global__ void __launch_bounds__((NCW + 1) * 32, NCW <= kPairTwoCtaNcw ? 2 : 1)
 batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restrict__ step_counter,
                     float* __restrict__ loss_hist, int hist_len, int iters, float* __restrict__ warp_loss,
-                    unsigned* ws, float* __restrict__ lpart) {
+                    unsigned* ws, float* __restrict__ light_part) {
+  float* lpart = GEN ? light_part : nullptr;
   constexpr int NT = NCW * 32;
   constexpr int TT = 2 * NT;                  // texels per tile
   constexpr int SLOT = kPairSlotPlanes * TT;  // floats per ring slot
@@ -2710,9 +2713,20 @@ int svbrdf_batched_steps(const void* device_plan, const void* host_plan, int los
   const int launches = h->light ? iters : (iters + kFuseMax - 1) / kFuseMax;
   for (int l = 0; l < launches; ++l) {
     const int k = iters / launches + (l < iters % launches ? 1 : 0);
-#define SVB_F(L, NCW, G)                                                                                       {                                                                                                              int prc = fuse_prepare<L, NCW, G>(ring);                                                                     if (prc) return prc;                                                                                         batched_fuse_kernel<L, NCW, G><<<h->n_ctas, (NCW + 1) * 32, fuse_smem<NCW>(ring), st>>>(                         plan, hyper, step_counter, loss_hist, hist_len, k, part, ws, lpart);                                   }
-#define SVB_FG(L, NCW)                  if (h->general) SVB_F(L, NCW, true)   else SVB_F(L, NCW, false)
-#define SVB_FL(NCW)                                         if (loss_kind == SVBRDF_LOSS_MSE) SVB_FG(0, NCW)          else if (loss_kind == SVBRDF_LOSS_LOG1P) SVB_FG(1, NCW)   else SVB_FG(2, NCW)
+#define SVB_F(L, NCW, G)                                                                              \
+  {                                                                                                   \
+    int prc = fuse_prepare<L, NCW, G>(ring);                                                          \
+    if (prc) return prc;                                                                              \
+    batched_fuse_kernel<L, NCW, G><<<h->n_ctas, (NCW + 1) * 32, fuse_smem<NCW>(ring), st>>>(          \
+        plan, hyper, step_counter, loss_hist, hist_len, k, part, ws, lpart);                          \
+  }
+#define SVB_FG(L, NCW)                                \
+  if (h->general || h->light) SVB_F(L, NCW, true)     \
+  else SVB_F(L, NCW, false)
+#define SVB_FL(NCW)                                       \
+  if (loss_kind == SVBRDF_LOSS_MSE) SVB_FG(0, NCW)        \
+  else if (loss_kind == SVBRDF_LOSS_LOG1P) SVB_FG(1, NCW) \
+  else SVB_FG(2, NCW)
     if (h->variant == 3) {
       switch (h->threads) {
         case 224: SVB_FL(7) break;
