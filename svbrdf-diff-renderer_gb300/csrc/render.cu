@@ -47,6 +47,7 @@ int device_sm_count() {
 // ------------------------------------------------------------------ kernels
 constexpr int kRenderThreads = 256;
 
+// Forward render with the image loss (Microfacet.render_loss), one texel per thread.
 template <int LOSS>
 __global__ void __launch_bounds__(kRenderThreads)
 render_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, const float* __restrict__ lit,
@@ -108,59 +109,119 @@ render_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, 
   }
 }
 
-template <bool GRAD_POW>
-__global__ void __launch_bounds__(kRenderThreads)
-render_bwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, const float* __restrict__ lit,
-                  const float* __restrict__ lpow, int V, int H, int W, float size,
-                  const float* __restrict__ gout, float* __restrict__ gtex, float* __restrict__ gpow,
-                  float4* partials, unsigned* counter, int B) {
+// ---- the forward render and its adjoint, one texel per thread
+//
+// Bound by HBM by their bytes (36 B of maps and 12 B per view a texel, and the adjoint's 36 B of
+// gradients), in practice by latency: a view of a texel is a chain of about 90 (forward) or 190
+// (adjoint) scalar instructions, which starts, in the adjoint, with its three gradients' loads.
+// The adjoint loads them one view ahead of their use, and a block takes chunks of kTexels texels,
+// material by material, instead of dividing every texel's index: 1024^2, 9 views, forward 50 ->
+// 43 us, adjoint 123 -> 95 us. Two texels per thread or per FP32x2 instruction take 30 and
+// 68 us, but round differently, and a change of rounding here passes through a whole TF32 generator
+// in the latent fit, so a texel's arithmetic stays texel_view's.
+constexpr int kTexels = 128;
+
+__global__ void __launch_bounds__(kTexels)
+render_texels_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, const float* __restrict__ lit,
+                         const float* __restrict__ lpow, int V, int H, int W, float size, float* __restrict__ out,
+                         int B) {
   __shared__ View s_views[kMaxViews];
   __shared__ float s_pow[3];
-  __shared__ float s_red[kRenderThreads / 32];
-  __shared__ double s_dred[4 * kRenderThreads / 32];
+  stage_views(s_views, cam, lit, V);
+  if (threadIdx.x < 3) s_pow[threadIdx.x] = lpow[threadIdx.x];
+  __syncthreads();
+  const int T = H * W;
+  const long long chunks = ((long long)T + kTexels - 1) / kTexels;
+  float unused = 0.f;
+  Adj dummy;
+  for (long long p = blockIdx.x; p < chunks * B; p += gridDim.x) {
+    const long long b = p / chunks, at = (p - b * chunks) * kTexels + threadIdx.x;
+    if (at >= T) continue;
+    const int idx = (int)at;
+    const float* texb = tex + 9LL * T * b + idx;
+    float* outb = out + 3LL * V * T * b + idx;
+    float t[9];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) t[c] = texb[(long long)c * T];
+    Maps m;
+    decode(t, m);
+    float px, py;
+    texel_pos(idx / W, idx % W, W, H, size, px, py);
+#pragma unroll 3
+    for (int v = 0; v < V; ++v) {
+      float io[3];
+      if (s_views[v].coloc != 0.f)
+        texel_view<kModeFwd, -1, false, true>(m, px, py, s_views[v], s_pow, io, unused, dummy);
+      else
+        texel_view<kModeFwd, -1, false, false>(m, px, py, s_views[v], s_pow, io, unused, dummy);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) outb[(3LL * v + c) * T] = io[c];
+    }
+  }
+}
+
+template <bool GRAD_POW>
+__global__ void __launch_bounds__(kTexels, GRAD_POW ? 4 : 5)
+render_texels_bwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, const float* __restrict__ lit,
+                         const float* __restrict__ lpow, int V, int H, int W, float size,
+                         const float* __restrict__ gout, float* __restrict__ gtex, float* __restrict__ gpow,
+                         float4* partials, unsigned* counter, int B) {
+  __shared__ View s_views[kMaxViews];
+  __shared__ float s_pow[3];
+  __shared__ float s_red[kTexels / 32];
+  __shared__ double s_dred[4 * kTexels / 32];
   __shared__ int s_flag;
   stage_views(s_views, cam, lit, V);
   if (threadIdx.x < 3) s_pow[threadIdx.x] = lpow[threadIdx.x];
   __syncthreads();
-
-  const long long T = (long long)H * W;
+  const int T = H * W;
+  const long long chunks = ((long long)T + kTexels - 1) / kTexels;
   float gp0 = 0.f, gp1 = 0.f, gp2 = 0.f, unused = 0.f;
-  for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < T * B;
-       gi += (long long)gridDim.x * blockDim.x) {
-    const long long b = gi / T, idx = gi - b * T;
-    const float* texb = tex + 9 * T * b;
+  for (long long p = blockIdx.x; p < chunks * B; p += gridDim.x) {
+    const long long b = p / chunks, at = (p - b * chunks) * kTexels + threadIdx.x;
+    if (at >= T) continue;
+    const int idx = (int)at;
+    const float* texb = tex + 9LL * T * b + idx;
+    const float* gb = gout + 3LL * V * T * b + idx;
+    float* gt = gtex + 9LL * T * b + idx;
+    float next[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) next[c] = gb[(long long)c * T];
     float t[9];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) t[c] = texb[c * T + idx];
+    for (int c = 0; c < 9; ++c) t[c] = texb[(long long)c * T];
     Maps m;
     decode(t, m);
     float px, py;
-    texel_pos((int)(idx / W), (int)(idx % W), W, H, size, px, py);
+    texel_pos(idx / W, idx % W, W, H, size, px, py);
     Adj a;
     adj_zero(a);
-    const long long vb = 3LL * V * T * b;
     for (int v = 0; v < V; ++v) {
-      float io[3];
+      float io[3] = {next[0], next[1], next[2]};
+      if (v + 1 < V) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) io[c] = gout[vb + (3LL * v + c) * T + idx];
+        for (int c = 0; c < 3; ++c) next[c] = gb[(3LL * (v + 1) + c) * T];
+      }
       if (s_views[v].coloc != 0.f)
         texel_view<kModeBwd, kLossMSE, GRAD_POW, true>(m, px, py, s_views[v], s_pow, io, unused, a);
       else
         texel_view<kModeBwd, kLossMSE, GRAD_POW, false>(m, px, py, s_views[v], s_pow, io, unused, a);
     }
+#pragma unroll
+    for (int c = 0; c < 9; ++c) t[c] = texb[(long long)c * T];  // again (L1 or L2) rather than live through the views
     float g[9];
     adj_to_params(t, m, a, 1.0f, g);
 #pragma unroll
-    for (int c = 0; c < 9; ++c) gtex[9 * T * b + c * T + idx] = g[c];
+    for (int c = 0; c < 9; ++c) gt[(long long)c * T] = g[c];
     if (GRAD_POW) { gp0 += a.gp[0]; gp1 += a.gp[1]; gp2 += a.gp[2]; }
   }
   if (GRAD_POW) {
-    const float b0 = block_sum<kRenderThreads>(gp0, s_red);
-    const float b1 = block_sum<kRenderThreads>(gp1, s_red);
-    const float b2 = block_sum<kRenderThreads>(gp2, s_red);
+    const float b0 = block_sum<kTexels>(gp0, s_red);
+    const float b1 = block_sum<kTexels>(gp1, s_red);
+    const float b2 = block_sum<kTexels>(gp2, s_red);
     if (publish_partial_and_check_last(partials, counter, make_float4(0.f, b0, b1, b2), &s_flag)) {
       double tot[4];
-      sum_partials<kRenderThreads>(partials, gridDim.x, tot, s_dred);
+      sum_partials<kTexels>(partials, gridDim.x, tot, s_dred);
       if (threadIdx.x == 0) {
         gpow[0] = (float)tot[1];
         gpow[1] = (float)tot[2];
@@ -190,6 +251,12 @@ int grid_for(long long T, int threads, int occupancy_blocks) {
   if (cap > kMaxGrid) cap = kMaxGrid;
   if (need > cap) need = cap;
   return (int)(need < 1 ? 1 : need);
+}
+
+// Blocks of the kernels above: one per chunk of a material, up to `most`.
+static int chunk_grid(long long T, int batch, long long most) {
+  const long long need = (T + kTexels - 1) / kTexels * batch;
+  return (int)(need < most ? need : most);
 }
 
 template <typename K>
@@ -244,7 +311,10 @@ int svbrdf_render_fwd_batch(const float* textures, const float* camera_pos, cons
                                                           partials, counter, loss_out, inv_n, batch);       \
     break;                                                                                                  \
   }
-    case SVBRDF_LOSS_NONE: SVB_FWD(-1)
+    case SVBRDF_LOSS_NONE:
+      render_texels_fwd_kernel<<<chunk_grid(T, batch, kMaxGrid), kTexels, 0, st>>>(textures, camera_pos, light_pos, light_pow,
+                                                                         n_views, height, width, size, out, batch);
+      break;
     case SVBRDF_LOSS_MSE: SVB_FWD(0)
     case SVBRDF_LOSS_LOG1P: SVB_FWD(1)
     default: SVB_FWD(2)
@@ -276,20 +346,19 @@ int svbrdf_render_bwd_batch(const float* textures, const float* camera_pos, cons
   unsigned* counter = (unsigned*)workspace;
   float4* partials = workspace ? (float4*)((char*)workspace + 16) : nullptr;
   cudaStream_t st = (cudaStream_t)stream;
-  if (grad_light_pow) {
-    static int occ = occupancy(render_bwd_kernel<true>, kRenderThreads);
-    const int grid = grid_for(T * batch, kRenderThreads, occ);
-    render_bwd_kernel<true><<<grid, kRenderThreads, 0, st>>>(textures, camera_pos, light_pos, light_pow, n_views,
+  // with the light power, as many blocks as the device holds at once: the last one sums a partial of
+  // each (2048 of them took 5 us of a 512^2 material's 31)
+  const int sms = device_sm_count();
+  const int grid = chunk_grid(T, batch, grad_light_pow && sms > 0 ? 4LL * sms : kMaxGrid);
+  if (grad_light_pow)
+    render_texels_bwd_kernel<true><<<grid, kTexels, 0, st>>>(textures, camera_pos, light_pos, light_pow, n_views,
                                                              height, width, size, grad_out, grad_textures,
                                                              grad_light_pow, partials, counter, batch);
-  } else {
-    static int occ = occupancy(render_bwd_kernel<false>, kRenderThreads);
-    const int grid = grid_for(T * batch, kRenderThreads, occ);
-    render_bwd_kernel<false><<<grid, kRenderThreads, 0, st>>>(textures, camera_pos, light_pos, light_pow, n_views,
-                                                              height, width, size, grad_out, grad_textures,
-                                                              nullptr, partials, counter, batch);
-  }
-  return check_launch("render_bwd_kernel");
+  else
+    render_texels_bwd_kernel<false><<<grid, kTexels, 0, st>>>(textures, camera_pos, light_pos, light_pow, n_views,
+                                                              height, width, size, grad_out, grad_textures, nullptr,
+                                                              partials, counter, batch);
+  return check_launch("render_texels_bwd_kernel");
 }
 
 int svbrdf_render_bwd(const float* textures, const float* camera_pos, const float* light_pos,

@@ -149,3 +149,40 @@ def test_batched_eval_matches_per_material(svb, golden, cuda):
         assert torch.equal(tb.grad[b:b + 1], t1.grad)
         g_sum += lp.grad
     assert rel_l2(g_batch, g_sum) <= 1e-6
+
+
+@pytest.mark.parametrize("res,views,batch", [(1, 1, 1), (3, 2, 2), (16, 9, 1), (17, 5, 3), (45, 16, 1), (46, 64, 2)])
+@pytest.mark.parametrize("coloc", [True, False])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_texel_chunks_match_fp64(svb, cuda, res, views, batch, coloc, shift):
+    """The forward and adjoint on texel counts around their chunks of 128 (one texel, a partly filled
+    last chunk, several chunks), materials and views, one view to the most, and tensors that start
+    4 bytes off an 8-byte boundary, against FP64 autograd: the tolerances of the tests above
+    (relative L2 1e-5 for renders, 1e-4 for gradients)."""
+    from oracle import microfacet_ref as R
+    g = torch.Generator().manual_seed(res * 100 + views)
+    tex = torch.rand(batch, 9, res, res, generator=g) * 1.4 - 0.7
+    cam = svb.scenes.random_views(views, g)
+    lit = cam.clone() if coloc else svb.scenes.random_views(views, g)
+    gout = torch.randn(batch * views, 3, res, res, generator=g)
+    lp = torch.tensor([1500.0, 1200.0, 1700.0])
+    outs, gtex, glight = [], [], torch.zeros(3, dtype=torch.float64)
+    for b in range(batch):
+        t, l = tex[b:b + 1].double().requires_grad_(True), lp.double().requires_grad_(True)
+        o = R.render(t, cam, lit, l, 17.0, torch.float64)
+        o.backward(gout[b * views:(b + 1) * views].double())
+        outs.append(o.detach()); gtex.append(t.grad); glight += l.grad
+    flat = torch.empty(tex.numel() + 1, device=cuda)
+    dt = flat[shift:shift + tex.numel()].view(tex.shape)
+    dt.copy_(tex)
+    gflat = torch.empty(gout.numel() + 1, device=cuda)
+    dg = gflat[shift:shift + gout.numel()].view(gout.shape)
+    dg.copy_(gout)
+    dt.requires_grad_(True)
+    dl = lp.to(cuda).requires_grad_(True)
+    r = svb.Microfacet(res, views, 17.0, [cam, lit, dl], cuda)
+    o = r.eval(dt)
+    got = torch.autograd.grad(o, [dt, dl], dg)
+    assert rel_l2(o.detach(), torch.cat(outs)) <= 1e-5
+    assert rel_l2(got[0], torch.cat(gtex)) <= 1e-4
+    assert rel_l2(got[1], glight) <= 1e-4
