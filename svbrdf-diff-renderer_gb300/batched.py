@@ -219,16 +219,16 @@ class BatchedOptim:
         """The device half of ``reset``: transform freshly uploaded targets for the loss, zero
         the moments, the step counter and the loss history (and, with ``optim_light``, put
         each light power back to its initial value with a fresh Adam state)."""
-        for i in range(self.n):
-            if new_targets and self.loss == "log1p":
-                self.tgt[i].log1p_()
-            self.m1[i].zero_()
-            self.m2[i].zero_()
-            if self.optim_light:
-                self.lpow[i].copy_(self.lpow0[i])
-                self.lstate[i].zero_()
+        if new_targets and self.loss == "log1p":
+            for t in self.tgt:
+                t.log1p_()
+        zero = [*self.m1, *self.m2, self.loss_hist]
+        if self.optim_light:
+            for p, p0 in zip(self.lpow, self.lpow0):
+                p.copy_(p0)
+            zero += self.lstate
+        torch._foreach_zero_(zero)  # one launch for all of them
         self.step_dev.zero_()
-        self.loss_hist.zero_()
         self.step_count = 0
 
     def textures(self, i: int) -> torch.Tensor:

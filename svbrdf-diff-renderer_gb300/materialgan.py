@@ -31,6 +31,8 @@ from typing import List, Optional
 import torch
 import torch.nn.functional as Fn
 
+from . import _native as N
+
 LRELU_GAIN = math.sqrt(2.0)
 
 
@@ -50,17 +52,21 @@ class _Dense(torch.nn.Module):
         self.lr_mul = lr_mul
         self.act = act
 
-    def forward(self, x):
+    def scaled(self):
+        """The run-time pair (weight x scale, bias x lr_mul); of frozen parameters computed once,
+        while they are unchanged."""
         if self.weight.requires_grad or self.bias.requires_grad:
-            w, b = self.weight * self.scale, self.bias * self.lr_mul
-        else:  # frozen: the scaled pair once, while the parameters are unchanged
-            key = (self.weight.data_ptr(), self.weight._version, self.bias.data_ptr(), self.bias._version,
-                   self.weight.dtype)
-            if getattr(self, "_scaled_key", None) != key:
-                with torch.no_grad():
-                    self._w_scaled, self._b_scaled = self.weight * self.scale, self.bias * self.lr_mul
-                self._scaled_key = key
-            w, b = self._w_scaled, self._b_scaled
+            return self.weight * self.scale, self.bias * self.lr_mul
+        key = (self.weight.data_ptr(), self.weight._version, self.bias.data_ptr(), self.bias._version,
+               self.weight.dtype)
+        if getattr(self, "_scaled_key", None) != key:
+            with torch.no_grad():
+                self._w_scaled, self._b_scaled = self.weight * self.scale, self.bias * self.lr_mul
+            self._scaled_key = key
+        return self._w_scaled, self._b_scaled
+
+    def forward(self, x):
+        w, b = self.scaled()
         y = Fn.linear(x, w, b)
         return Fn.leaky_relu(y, 0.2) * LRELU_GAIN if self.act else y
 
@@ -117,8 +123,6 @@ class _Upsample2Cuda(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x):
-        from . import _native as N
-
         L = N.lib()
         x = x.contiguous()
         b, c, h, w = x.shape
@@ -129,8 +133,6 @@ class _Upsample2Cuda(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         L = N.lib()
         b, c, h, w = ctx.hw
         g = g.contiguous()
@@ -174,7 +176,7 @@ def _is_nhwc(x):
 
 
 def _cl(t):
-    return t.contiguous(memory_format=CL)
+    return t if t.is_contiguous(memory_format=CL) else t.contiguous(memory_format=CL)
 
 
 class _UpsampleNHWC(torch.autograd.Function):
@@ -185,8 +187,6 @@ class _UpsampleNHWC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, s, halo=0):
-        from . import _native as N
-
         x = _cl(x)
         s = s.contiguous() if s is not None else None
         b, c, h, w = x.shape
@@ -200,8 +200,6 @@ class _UpsampleNHWC(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         x, s = ctx.saved_tensors
         b, c, h, w = x.shape
         L, st = N.lib(), N.stream_handle(x.device)
@@ -236,8 +234,6 @@ def generator_device_error(device="cuda") -> int:
 
 def _conv_tf32(x, w, y, b, h, wd, cin, cout, k, pad):
     """One svbrdf_gen_conv_tf32_ex call; maps with few tiles split K over a workspace."""
-    from . import _native as N
-
     L = N.lib()
     nb = int(L.svbrdf_gen_conv_tf32_ws_bytes(b, h, wd, cin, cout, k, pad))
     ws = torch.empty(nb, device=x.device, dtype=torch.uint8) if nb > 0 else None
@@ -255,8 +251,6 @@ class _ConvTF32(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w_fwd, w_dg, cout, k, pad, keep_pad=False):
-        from . import _native as N
-
         x = _cl(x)
         b, c, h, wd = x.shape
         coutp = w_fwd.shape[0]
@@ -270,8 +264,6 @@ class _ConvTF32(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gy):
-        from . import _native as N
-
         (w_dg,) = ctx.saved_tensors
         b, c, h, wd, coutp, cout, k, pad, ho, wo = ctx.geom
         if coutp != cout and not ctx.keep_pad:
@@ -292,8 +284,6 @@ class _ActScaleNHWC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, d, noise, ns, bias, gain, s2):
-        from . import _native as N
-
         y, d, bias, s2 = _cl(y), d.contiguous(), bias.contiguous(), s2.contiguous()
         noise = noise.contiguous() if noise is not None else None
         b, c, h, w = y.shape
@@ -308,8 +298,6 @@ class _ActScaleNHWC(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         y, d, noise, ns, bias, s2 = ctx.saved_tensors
         b, c, h, w = y.shape
         L = N.lib()
@@ -337,8 +325,6 @@ class _RgbNHWC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, yp, bias, prev, c):
-        from . import _native as N
-
         b, cp, h, w = yp.shape
         img = torch.empty(b, c, h, w, device=yp.device, dtype=torch.float32)
         N.check(N.lib().svbrdf_gen_rgb_nhwc(yp.data_ptr(), cp, bias.data_ptr(), N.ptr(prev), img.data_ptr(), b, c, h, w,
@@ -348,8 +334,6 @@ class _RgbNHWC(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         b, cp, c, h, w, has_prev = ctx.geom
         L = N.lib()
         st = N.stream_handle(g.device)
@@ -368,8 +352,6 @@ class _ScaleNHWC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, s):
-        from . import _native as N
-
         x, s = _cl(x), s.contiguous()
         b, c, h, w = x.shape
         y = torch.empty_like(x)
@@ -380,8 +362,6 @@ class _ScaleNHWC(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         x, s = ctx.saved_tensors
         b, c, h, w = x.shape
         L = N.lib()
@@ -400,8 +380,6 @@ class _ActNHWC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, d, noise, ns, bias, gain):
-        from . import _native as N
-
         y, d, bias = _cl(y), d.contiguous(), bias.contiguous()
         noise = noise.contiguous() if noise is not None else None
         b, c, h, w = y.shape
@@ -415,8 +393,6 @@ class _ActNHWC(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         y, d, noise, ns, bias = ctx.saved_tensors
         b, c, h, w = y.shape
         L = N.lib()
@@ -434,14 +410,35 @@ class _ActNHWC(torch.autograd.Function):
         return gy, gd, gn, None, None, None
 
 
+class _StyleDemod(torch.autograd.Function):
+    """A frozen layer's style s = affine(w) and demodulation d = rsqrt(s^2 w2t + 1e-8) (None
+    without): ``a`` [cin, w_dim] and ``bias`` are the scaled affine pair, ``w2t`` [cin, cout] the
+    squared sums of the scaled weight. The forward is the operations that the modules would run; the
+    adjoint, gw = (gs - s ((gd d^3) w2t^T)) a, is five operations where autograd runs a node, with its
+    own launches, for each of linear, pow, mm, add and rsqrt."""
+
+    @staticmethod
+    def forward(ctx, w, a, bias, w2t):
+        s = Fn.linear(w, a, bias)
+        d = torch.rsqrt(s.pow(2) @ w2t + 1e-8) if w2t is not None else None
+        ctx.save_for_backward(s, d, a, w2t)
+        return s, d
+
+    @staticmethod
+    def backward(ctx, gs, gd):
+        s, d, a, w2t = ctx.saved_tensors
+        if gd is not None and d is not None:
+            gq = torch.mm(gd * (d * d * d), w2t.t())
+            gs = s * gq.neg_() if gs is None else torch.addcmul(gs, s, gq, value=-1.0)
+        return (gs @ a if gs is not None else None), None, None, None
+
+
 class _ScaleCuda(torch.autograd.Function):
     """x[b, c] * s[b, c] (a modulated conv's input scaling) as one kernel each way; the
     backward also forms the style gradient sum_hw g x per plane (svbrdf_gen_scale[_bwd])."""
 
     @staticmethod
     def forward(ctx, x, s):
-        from . import _native as N
-
         x, s = x.contiguous(), s.contiguous()
         b, c, h, w = x.shape
         y = torch.empty_like(x)
@@ -452,8 +449,6 @@ class _ScaleCuda(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         x, s = ctx.saved_tensors
         b, c, h, w = x.shape
         g = g.contiguous()
@@ -471,8 +466,6 @@ class _ActCuda(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, d, noise, ns, bias, gain):
-        from . import _native as N
-
         y, d, bias = y.contiguous(), d.contiguous(), bias.contiguous()
         noise = noise.contiguous() if noise is not None else None
         b, c, h, w = y.shape
@@ -486,8 +479,6 @@ class _ActCuda(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        from . import _native as N
-
         y, d, noise, ns, bias = ctx.saved_tensors
         b, c, h, w = y.shape
         g = g.contiguous()
@@ -555,8 +546,10 @@ class _ModConv(torch.nn.Module):
         is this layer's (style, demodulation) pair when the generator computed them for all
         layers at once (StyleGAN2Generator._styles); ``prescaled`` says that the
         channels-last input already carries this layer's style scaling (_ActScaleNHWC)."""
-        s = self.affine(w) if sd is None else sd[0]  # [B, cin]
         wsc, w2t = self._scaled_weight()
+        if sd is None:
+            sd = self._style(w, w2t)
+        s, d = sd  # [B, cin], [B, cout] or None
         # an up-sampling layer convolves the up-sampled map with its one-sample halo, unpadded
         # (_upsample2_halo): the reference's transposed convolution + filter on the border too
         pad = 0 if self.up else self.k // 2
@@ -576,10 +569,16 @@ class _ModConv(torch.nn.Module):
             if self.up:
                 x = _upsample2_halo(x)  # per-channel linear: commutes with the channel scaling
             y = Fn.conv2d(x, wsc, padding=pad)
-        d = None
-        if self.demod:
-            d = torch.rsqrt(s.pow(2) @ w2t + 1e-8) if sd is None else sd[1]  # [B, cout]
         return y, d
+
+    def _style(self, w, w2t):
+        """(style, demodulation or None) of w [B, w_dim]."""
+        aff = self.affine
+        if (_use_kernels(w) and w.dim() == 2 and aff.weight.dtype == torch.float32 and not aff.act and
+                not (self.weight.requires_grad or aff.weight.requires_grad or aff.bias.requires_grad)):
+            return _StyleDemod.apply(w, *aff.scaled(), w2t if self.demod else None)
+        s = aff(w)
+        return s, (torch.rsqrt(s.pow(2) @ w2t + 1e-8) if self.demod else None)
 
     def _scaled_weight(self):
         """(scale * weight, its squared sums over the taps transposed, [cin, cout]). A frozen

@@ -24,35 +24,33 @@ def _as_dev(x, device):
 class _RenderFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, textures, light_pow, r):
-        L = N.lib()
-        tex = textures.detach().to(torch.float32).contiguous()
-        lp = light_pow.detach().to(torch.float32).contiguous()
+        tex, lp = N.plain(textures), N.plain(light_pow)
         B, _, H, W = tex.shape
-        out = torch.empty(B * r.n_of_imgs, 3, H, W, device=tex.device, dtype=torch.float32)
-        s = N.stream_handle(tex.device)
+        device = tex.device
+        out = torch.empty((B * r.n_of_imgs, 3, H, W), device=device, dtype=torch.float32)
         # the whole batch in one launch
-        N.check(L.svbrdf_render_fwd_batch(tex.data_ptr(), r._cam.data_ptr(), r._lit.data_ptr(), lp.data_ptr(),
-                                          r.n_of_imgs, H, W, float(r.size), B, out.data_ptr(), None, -1, None, None,
-                                          0, s))
+        N.check(N.lib().svbrdf_render_fwd_batch(tex.data_ptr(), r._cam.data_ptr(), r._lit.data_ptr(), lp.data_ptr(),
+                                                r.n_of_imgs, H, W, float(r.size), B, out.data_ptr(), None, -1, None, None, 0,
+                                                N.stream_handle(device)))
         ctx.save_for_backward(tex, lp)
         ctx.r = r
         return out
 
     @staticmethod
     def backward(ctx, gout):
-        L = N.lib()
         tex, lp = ctx.saved_tensors
         r = ctx.r
-        gout = gout.to(torch.float32).contiguous()
+        gout = N.plain(gout)
         B, _, H, W = tex.shape
+        device = tex.device
         gtex = torch.empty_like(tex)
-        want_pow = ctx.needs_input_grad[1]
-        gpow = torch.zeros(3, device=tex.device, dtype=torch.float32) if want_pow else None
-        s = N.stream_handle(tex.device)
+        # the kernel writes all three sums
+        gpow = torch.empty(3, device=device, dtype=torch.float32) if ctx.needs_input_grad[1] else None
         # the whole batch in one launch; the light-power gradient sums over all of it
-        N.check(L.svbrdf_render_bwd_batch(tex.data_ptr(), r._cam.data_ptr(), r._lit.data_ptr(), lp.data_ptr(),
-                                          r.n_of_imgs, H, W, float(r.size), B, gout.data_ptr(), gtex.data_ptr(),
-                                          N.ptr(gpow), r._workspace.data_ptr(), r._workspace.numel(), s))
+        N.check(N.lib().svbrdf_render_bwd_batch(tex.data_ptr(), r._cam.data_ptr(), r._lit.data_ptr(), lp.data_ptr(),
+                                                r.n_of_imgs, H, W, float(r.size), B, gout.data_ptr(), gtex.data_ptr(),
+                                                N.ptr(gpow), r._workspace.data_ptr(), r._workspace_bytes,
+                                                N.stream_handle(device)))
         return gtex, gpow, None
 
 
@@ -80,7 +78,8 @@ class Microfacet:
         self.light_pow = lp if torch.is_tensor(lp) and lp.device == self.device else _as_dev(lp, self.device)
         if self.n_of_imgs > N.load().svbrdf_max_views():
             raise ValueError(f"n={self.n_of_imgs} views exceeds the kernel maximum {N.load().svbrdf_max_views()}")
-        self._workspace = torch.zeros(int(N.load().svbrdf_workspace_bytes()), dtype=torch.uint8, device=self.device)
+        self._workspace_bytes = int(N.load().svbrdf_workspace_bytes())
+        self._workspace = torch.zeros(self._workspace_bytes, dtype=torch.uint8, device=self.device)
 
     @property
     def camera_pos(self):

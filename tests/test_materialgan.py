@@ -530,3 +530,37 @@ def test_gpu_generator_tf32_matches_reference_network(svb, cuda):
           + ", ".join(f"{e:.2e}" for e in ours) + "; cuDNN TF32 " + ", ".join(f"{e:.2e}" for e in lib))
     for e, e_lib, floor in zip(ours, lib, (1e-2, 3e-2, 3e-2)):
         assert e <= max(floor, 2 * e_lib)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,cin,cout", [(1, 12, 10), (3, 64, 40), (16, 512, 256)])
+@pytest.mark.parametrize("demod", [True, False])
+def test_style_demod_node_matches_autograd(svb, cuda, batch, cin, cout, demod):
+    """The frozen layer's style and demodulation as one autograd node against autograd of the same
+    operations in FP64: values and the gradient of w, from both outputs and from either alone.
+    Five FP32 operations over sums of up to 512 terms: relative L2 within 1e-5."""
+    MG = svb.materialgan
+    g = torch.Generator().manual_seed(cin)
+    conv = MG._ModConv(cin, cout, 3, 24, g, demod=demod)
+    for p in conv.parameters():
+        p.requires_grad_(False)
+    w = torch.randn(batch, 24, generator=g)
+    gs, gd = torch.randn(batch, cin, generator=g), torch.randn(batch, cout, generator=g)
+    ref = MG._ModConv(cin, cout, 3, 24, torch.Generator().manual_seed(0), demod=demod).double()
+    ref.load_state_dict({k: v.double() for k, v in conv.state_dict().items()})
+    wr = w.double().requires_grad_(True)
+    sr = ref.affine(wr)
+    dr = torch.rsqrt(sr.pow(2) @ ref._scaled_weight()[1] + 1e-8)
+    conv = conv.to(cuda)
+    wd = w.to(cuda).requires_grad_(True)
+    s, d = conv._style(wd, conv._scaled_weight()[1])
+    assert rel_l2(s.detach(), sr.detach()) <= 1e-5
+    assert (d is None) == (not demod)
+    pairs = [((s,), (gs,), (sr,))]
+    if demod:
+        assert rel_l2(d.detach(), dr.detach()) <= 1e-5
+        pairs += [((d,), (gd,), (dr,)), ((s, d), (gs, gd), (sr, dr))]
+    for out, gr, outr in pairs:
+        got = torch.autograd.grad(out, wd, [t.to(cuda) for t in gr], retain_graph=True)[0]
+        want = torch.autograd.grad(outr, wr, [t.double() for t in gr], retain_graph=True)[0]
+        assert rel_l2(got, want) <= 1e-5
