@@ -170,6 +170,8 @@ def _declare(L):
     L.svbrdf_gen_conv_tf32_ws_bytes.argtypes = [I, I, I, I, I, I, I]
     L.svbrdf_gen_conv_tf32_ex.restype = I
     L.svbrdf_gen_conv_tf32_ex.argtypes = [P, P, P, P, ctypes.c_longlong, I, I, I, I, I, I, I, P, P]
+    L.svbrdf_gen_conv_act_tf32.restype = I
+    L.svbrdf_gen_conv_act_tf32.argtypes = [P, P, P, P, ctypes.c_longlong, I, I, I, I, I, I, I, P, P, P, P, F, P, P, P, P]
     L.svbrdf_gen_upsample2.restype = I
     L.svbrdf_gen_upsample2.argtypes = [P, P, ctypes.c_longlong, I, I, P]
     L.svbrdf_gen_upsample2_scaled.restype = I
@@ -241,6 +243,7 @@ EXPORTS = [
     "svbrdf_gen_scale_nhwc", "svbrdf_gen_scale_nhwc_bwd", "svbrdf_gen_act_nhwc", "svbrdf_gen_act_nhwc_bwd",
     "svbrdf_gen_act_scale_nhwc", "svbrdf_gen_act_scale_nhwc_bwd",
     "svbrdf_gen_conv_tf32", "svbrdf_gen_conv_tf32_ws_bytes", "svbrdf_gen_conv_tf32_ex",
+    "svbrdf_gen_conv_act_tf32",
     "svbrdf_envmap_render", "svbrdf_selftest_wait_timeout",
 ]
 

@@ -277,6 +277,50 @@ class _ConvTF32(torch.autograd.Function):
         return gx, None, None, None, None, None, None
 
 
+class _ConvActTF32(torch.autograd.Function):
+    """_ConvTF32 of a 3x3 layer followed by its epilogue, _ActNHWC or with ``s2`` _ActScaleNHWC, in one
+    call (svbrdf_gen_conv_act_tf32): one pass over the output where the convolution's halo form runs.
+    The adjoint is theirs: the epilogue's, then the data gradient."""
+
+    @staticmethod
+    def forward(ctx, x, w_fwd, w_dg, pad, d, noise, ns, bias, gain, s2):
+        x, d, bias = _cl(x), d.contiguous(), bias.contiguous()
+        noise = noise.contiguous() if noise is not None else None
+        s2 = s2.contiguous() if s2 is not None else None
+        b, c, h, wd = x.shape
+        cout = w_fwd.shape[0]
+        ho, wo = h + 2 * pad - 2, wd + 2 * pad - 2
+        y = torch.empty((b, cout, ho, wo), device=x.device, dtype=torch.float32, memory_format=CL)
+        out = torch.empty_like(y)
+        L = N.lib()
+        nb = L.svbrdf_gen_conv_tf32_ws_bytes(b, h, wd, c, cout, 3, pad)
+        ws = torch.empty(nb, device=x.device, dtype=torch.uint8) if nb > 0 else None
+        N.check(L.svbrdf_gen_conv_act_tf32(x.data_ptr(), w_fwd.data_ptr(), y.data_ptr(), N.ptr(ws), max(nb, 0), b, h,
+                                           wd, c, cout, 3, pad, d.data_ptr(), N.ptr(noise),
+                                           ns.data_ptr() if noise is not None else None, bias.data_ptr(), gain,
+                                           N.ptr(s2), out.data_ptr(), _tf32_err(x.device).data_ptr(),
+                                           N.stream_handle(x.device)))
+        ctx.save_for_backward(y, d, noise, ns, bias, s2, w_dg)
+        ctx.gain = gain
+        ctx.geom = (b, c, h, wd, cout, pad, ho, wo)
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        y, d, noise, ns, bias, s2, w_dg = ctx.saved_tensors
+        b, c, h, wd, cout, pad, ho, wo = ctx.geom
+        want_noise = noise is not None and ctx.needs_input_grad[5]
+        if s2 is None:
+            gy, gd, gn, gs2 = *_act_nhwc_bwd(_cl(g), y, d, noise, ns, bias, ctx.gain, want_noise), None
+        else:
+            gy, gd, gn, gs2 = _act_scale_nhwc_bwd(_cl(g), y, d, noise, ns, bias, ctx.gain, s2, want_noise)
+        gx = None
+        if ctx.needs_input_grad[0]:
+            gx = torch.empty((b, c, h, wd), device=g.device, dtype=torch.float32, memory_format=CL)
+            _conv_tf32(gy, w_dg, gx, b, ho, wo, cout, c, 3, 2 - pad)
+        return gx, None, None, None, gd, gn, None, None, None, gs2
+
+
 class _ActScaleNHWC(torch.autograd.Function):
     """_ActNHWC followed by the next layer's input scaling (x s2[b, c]) in one pass each way
     (svbrdf_gen_act_scale_nhwc[_bwd]), for an output whose only consumer is that layer: the
@@ -299,23 +343,42 @@ class _ActScaleNHWC(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         y, d, noise, ns, bias, s2 = ctx.saved_tensors
-        b, c, h, w = y.shape
-        L = N.lib()
-        g = _cl(g)
-        gy = torch.empty_like(y)
-        gd = torch.empty(b, c, device=y.device, dtype=torch.float32)
-        gs2 = torch.empty(b, c, device=y.device, dtype=torch.float32)
         want_noise = noise is not None and ctx.needs_input_grad[2]
-        gn = torch.empty_like(noise) if want_noise else None
-        nparts = L.svbrdf_gen_nhwc_partial_floats(b, c)
-        part = torch.empty(nparts, device=y.device, dtype=torch.float32)
-        part2 = torch.empty(nparts, device=y.device, dtype=torch.float32)
-        N.check(L.svbrdf_gen_act_scale_nhwc_bwd(g.data_ptr(), y.data_ptr(), d.data_ptr(), N.ptr(noise),
-                                                ns.data_ptr() if noise is not None else None, bias.data_ptr(), ctx.gain,
-                                                s2.data_ptr(), gy.data_ptr(), gd.data_ptr(), gs2.data_ptr(), N.ptr(gn),
-                                                part.data_ptr(), part2.data_ptr(), b, h * w, c,
-                                                N.stream_handle(y.device)))
+        gy, gd, gn, gs2 = _act_scale_nhwc_bwd(_cl(g), y, d, noise, ns, bias, ctx.gain, s2, want_noise)
         return gy, gd, gn, None, None, None, gs2
+
+
+def _act_scale_nhwc_bwd(g, y, d, noise, ns, bias, gain, s2, want_noise):
+    """(gy, gd, gnoise or None, gs2) of the epilogue with the next layer's scale."""
+    b, c, h, w = y.shape
+    L = N.lib()
+    gy = torch.empty_like(y)
+    gd = torch.empty(b, c, device=y.device, dtype=torch.float32)
+    gs2 = torch.empty(b, c, device=y.device, dtype=torch.float32)
+    gn = torch.empty_like(noise) if want_noise else None
+    nparts = L.svbrdf_gen_nhwc_partial_floats(b, c)
+    part = torch.empty(2 * nparts, device=y.device, dtype=torch.float32)
+    N.check(L.svbrdf_gen_act_scale_nhwc_bwd(g.data_ptr(), y.data_ptr(), d.data_ptr(), N.ptr(noise),
+                                            ns.data_ptr() if noise is not None else None, bias.data_ptr(), gain,
+                                            s2.data_ptr(), gy.data_ptr(), gd.data_ptr(), gs2.data_ptr(), N.ptr(gn),
+                                            part.data_ptr(), part.data_ptr() + 4 * nparts, b, h * w, c,
+                                            N.stream_handle(y.device)))
+    return gy, gd, gn, gs2
+
+
+def _act_nhwc_bwd(g, y, d, noise, ns, bias, gain, want_noise):
+    """(gy, gd, gnoise or None) of the style layer's epilogue."""
+    b, c, h, w = y.shape
+    L = N.lib()
+    gy = torch.empty_like(y)
+    gd = torch.empty(b, c, device=y.device, dtype=torch.float32)
+    gn = torch.empty_like(noise) if want_noise else None
+    part = torch.empty(L.svbrdf_gen_nhwc_partial_floats(b, c), device=y.device, dtype=torch.float32)
+    N.check(L.svbrdf_gen_act_nhwc_bwd(g.data_ptr(), y.data_ptr(), d.data_ptr(), N.ptr(noise),
+                                      ns.data_ptr() if noise is not None else None, bias.data_ptr(), gain,
+                                      gy.data_ptr(), gd.data_ptr(), N.ptr(gn), part.data_ptr(), b, h * w, c,
+                                      N.stream_handle(y.device)))
+    return gy, gd, gn
 
 
 class _RgbNHWC(torch.autograd.Function):
@@ -394,19 +457,8 @@ class _ActNHWC(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         y, d, noise, ns, bias = ctx.saved_tensors
-        b, c, h, w = y.shape
-        L = N.lib()
-        g = _cl(g)
-        gy = torch.empty_like(y)
-        gd = torch.empty(b, c, device=y.device, dtype=torch.float32)
         want_noise = noise is not None and ctx.needs_input_grad[2]
-        gn = torch.empty_like(noise) if want_noise else None
-        part = torch.empty(L.svbrdf_gen_nhwc_partial_floats(b, c), device=y.device, dtype=torch.float32)
-        N.check(L.svbrdf_gen_act_nhwc_bwd(g.data_ptr(), y.data_ptr(), d.data_ptr(),
-                                          noise.data_ptr() if noise is not None else None,
-                                          ns.data_ptr() if noise is not None else None, bias.data_ptr(), ctx.gain,
-                                          gy.data_ptr(), gd.data_ptr(), gn.data_ptr() if want_noise else None,
-                                          part.data_ptr(), b, h * w, c, N.stream_handle(y.device)))
+        gy, gd, gn = _act_nhwc_bwd(_cl(g), y, d, noise, ns, bias, ctx.gain, want_noise)
         return gy, gd, gn, None, None, None
 
 
@@ -546,6 +598,19 @@ class _ModConv(torch.nn.Module):
         is this layer's (style, demodulation) pair when the generator computed them for all
         layers at once (StyleGAN2Generator._styles); ``prescaled`` says that the
         channels-last input already carries this layer's style scaling (_ActScaleNHWC)."""
+        x, d, wsc, pad = self._input(x, w, sd, prescaled)
+        if _use_kernels(x) and _is_nhwc(x):
+            if self._tf32_ok(x):
+                w_fwd, w_dg = self._tf32_weights(wsc)
+                y = _ConvTF32.apply(x, w_fwd, w_dg, self.weight.shape[0], self.k, pad, keep_pad)
+            else:
+                y = Fn.conv2d(x, _cl(wsc), padding=pad)
+        else:
+            y = Fn.conv2d(x, wsc, padding=pad)
+        return y, d
+
+    def _input(self, x, w, sd, prescaled):
+        """(the convolution's style-scaled, up-sampled input, demodulation, scaled weight, padding)."""
         wsc, w2t = self._scaled_weight()
         if sd is None:
             sd = self._style(w, w2t)
@@ -559,17 +624,11 @@ class _ModConv(torch.nn.Module):
                 x = _UpsampleNHWC.apply(x, s, 1)
             elif not prescaled:
                 x = _ScaleNHWC.apply(x, s)
-            if self._tf32_ok(x):
-                w_fwd, w_dg = self._tf32_weights(wsc)
-                y = _ConvTF32.apply(x, w_fwd, w_dg, self.weight.shape[0], self.k, pad, keep_pad)
-            else:
-                y = Fn.conv2d(x, _cl(wsc), padding=pad)
         else:
             x = _ScaleCuda.apply(x, s) if _use_kernels(x) else x * s[:, :, None, None]
             if self.up:
                 x = _upsample2_halo(x)  # per-channel linear: commutes with the channel scaling
-            y = Fn.conv2d(x, wsc, padding=pad)
-        return y, d
+        return x, d, wsc, pad
 
     def _style(self, w, w2t):
         """(style, demodulation or None) of w [B, w_dim]."""
@@ -613,7 +672,16 @@ class _StyleLayer(torch.nn.Module):
         """``s_next``: the next layer's style, to scale this layer's output by in the same pass
         (channels-last kernel path only; the caller then passes ``prescaled`` to that layer)."""
         if self.kernel_ok(x, noise):
-            y, d = self.conv.parts(x, w, sd=sd, prescaled=prescaled)
+            conv = self.conv
+            if _is_nhwc(x) and conv.k == 3 and conv.weight.shape[0] % 32 == 0:
+                xs, d, wsc, pad = conv._input(x, w, sd, prescaled)
+                if _is_nhwc(xs) and d is not None and conv._tf32_ok(xs):
+                    w_fwd, w_dg = conv._tf32_weights(wsc)
+                    return _ConvActTF32.apply(xs, w_fwd, w_dg, pad, d, noise, self.noise_strength, self.bias,
+                                              LRELU_GAIN, s_next)
+                y = Fn.conv2d(xs, _cl(wsc), padding=pad)
+            else:
+                y, d = conv.parts(x, w, sd=sd, prescaled=prescaled)
             if s_next is not None and _is_nhwc(y):
                 return _ActScaleNHWC.apply(y, d, noise, self.noise_strength, self.bias, LRELU_GAIN, s_next)
             act = _ActNHWC if _is_nhwc(y) else _ActCuda
@@ -630,16 +698,20 @@ class _ToRGB(torch.nn.Module):
         self.conv = _ModConv(cin, cout, 1, w_dim, g, demod=False)
         self.bias = torch.nn.Parameter(torch.zeros(cout))
 
-    def forward(self, x, w, skip, sd=None):
+    def kernel_ok(self, x, skip) -> bool:
+        """Whether forward takes the fused path: the TF32 convolution's padded channels-last output,
+        bias and the up-sampled skip image in one pass that writes the image in NCHW."""
         cout = self.bias.shape[0]
-        if (_use_kernels(x) and _is_nhwc(x) and not self.bias.requires_grad and self.conv._tf32_ok(x) and
+        return (_use_kernels(x) and _is_nhwc(x) and not self.bias.requires_grad and self.conv._tf32_ok(x) and
                 x.shape[-1] % 2 == 0 and x.shape[-2] % 2 == 0 and
                 (skip is None or (skip.is_contiguous() and skip.dtype == torch.float32 and
-                                  tuple(skip.shape) == (x.shape[0], cout, x.shape[-2] // 2, x.shape[-1] // 2)))):
-            # the TF32 convolution's padded channels-last output, bias and the up-sampled skip
-            # image in one pass that writes the image in NCHW
-            yp, _ = self.conv.parts(x, w, keep_pad=True, sd=sd)
-            return _RgbNHWC.apply(_cl(yp), self.bias, skip, cout)
+                                  tuple(skip.shape) == (x.shape[0], cout, x.shape[-2] // 2, x.shape[-1] // 2))))
+
+    def forward(self, x, w, skip, sd=None, prescaled=False):
+        """``prescaled``: x carries this layer's style scaling already (kernel_ok inputs only)."""
+        if self.kernel_ok(x, skip):
+            yp, _ = self.conv.parts(x, w, keep_pad=True, sd=sd, prescaled=prescaled)
+            return _RgbNHWC.apply(_cl(yp), self.bias, skip, self.bias.shape[0])
         y = self.conv(x, w) + self.bias.view(1, -1, 1, 1)
         return y if skip is None else y + _upsample2(skip)
 
@@ -811,13 +883,18 @@ class StyleGAN2Generator(torch.nn.Module):
             # channels-last kernel path its epilogue also applies that layer's style scaling
             fuse = (bool(sd) and _is_nhwc(x) and up.kernel_ok(x, n_up) and conv.kernel_ok(x, n_conv)
                     and conv.conv in sd)
+            last = False
             if fuse:
                 x = up(x, wp[:, 1 + 2 * i], n_up, sd.get(up.conv), s_next=sd[conv.conv][0])
-                x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv), prescaled=True)
+                # the last map feeds only its toRGB layer: its epilogue applies that style too, and
+                # the unscaled map is neither stored nor read again
+                last = i == len(self.ups) - 1 and rgb.conv in sd and rgb.kernel_ok(x, img)
+                x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv), prescaled=True,
+                         s_next=sd[rgb.conv][0] if last else None)
             else:
                 x = up(x, wp[:, 1 + 2 * i], n_up, sd.get(up.conv))
                 x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv))
-            img = rgb(x, wp[:, 3 + 2 * i], img, sd.get(rgb.conv))
+            img = rgb(x, wp[:, 3 + 2 * i], img, sd.get(rgb.conv), prescaled=last)
         return img
 
 

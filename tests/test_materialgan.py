@@ -564,3 +564,46 @@ def test_style_demod_node_matches_autograd(svb, cuda, batch, cin, cout, demod):
         got = torch.autograd.grad(out, wd, [t.to(cuda) for t in gr], retain_graph=True)[0]
         want = torch.autograd.grad(outr, wr, [t.double() for t in gr], retain_graph=True)[0]
         assert rel_l2(got, want) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 32, 32, 16, 8), (1, 64, 32, 33, 17), (3, 128, 128, 32, 16), (2, 32, 256, 18, 24),
+                                   (16, 64, 512, 16, 16), (2, 64, 64, 8, 8), (1, 512, 512, 4, 4), (1, 64, 128, 47, 9)])
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("with_noise,scale", [(True, True), (False, False)])
+def test_conv_act_equals_its_two_kernels(svb, cuda, shape, pad, with_noise, scale):
+    """The convolution with the style layer's epilogue in one call against the two kernels, forward
+    and backward, over every patch form (halo tiles of one and two M-tiles and their clipped edges,
+    the split-K and stacked-image forms that run the epilogue kernel): the same arithmetic, so equal."""
+    MG = svb.materialgan
+    b, cin, cout, h, w = shape
+    ho, wo = h + 2 * pad - 2, w + 2 * pad - 2
+    if min(ho, wo) < 4:
+        pytest.skip("output narrower than 4")
+    g = torch.Generator(device=cuda).manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    cl = lambda t: t.contiguous(memory_format=torch.channels_last)
+    x = cl(rnd(b, cin, h, w))
+    wt = rnd(cout, cin, 3, 3) / (9 * cin) ** 0.5
+    w_fwd = wt.permute(0, 2, 3, 1).reshape(cout, 9, cin).contiguous()
+    w_dg = wt.flip(2, 3).permute(1, 2, 3, 0).reshape(cin, 9, cout).contiguous()
+    d, bias, s2 = rnd(b, cout), rnd(cout), rnd(b, cout) if scale else None
+    noise = rnd(b, 1, ho, wo) if with_noise else None
+    ns = torch.tensor(0.3, device=cuda)
+    go = cl(rnd(b, cout, ho, wo))
+    res = []
+    for fused in (True, False):
+        leaves = [t.clone(memory_format=torch.preserve_format).requires_grad_(True) if t is not None else None
+                  for t in (x, d, noise, s2)]
+        xl, dl, nl, sl = leaves
+        if fused:
+            out = MG._ConvActTF32.apply(xl, w_fwd, w_dg, pad, dl, nl, ns, bias, 1.25, sl)
+        else:
+            y = MG._ConvTF32.apply(xl, w_fwd, w_dg, cout, 3, pad, False)
+            out = (MG._ActScaleNHWC.apply(y, dl, nl, ns, bias, 1.25, sl) if scale
+                   else MG._ActNHWC.apply(y, dl, nl, ns, bias, 1.25))
+        wrt = [t for t in leaves if t is not None]
+        res.append([out.detach(), *torch.autograd.grad(out, wrt, go)])
+    assert MG.generator_device_error(cuda) == 0
+    for a, c in zip(*res):
+        assert torch.equal(a, c)
