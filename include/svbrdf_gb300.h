@@ -273,6 +273,15 @@ int svbrdf_desc_loss_sums(const float* buf, int n_segs, const long long* offsets
 int svbrdf_desc_conv1_fwd(const float* renders, const float* weight, const float* bias, float* out_f32,
                           void* out_bf16, int v, int h, int w, int downsample, void* stream);
 
+/* svbrdf_desc_conv1_fwd with the feature term of its hook in place of the FP32 features: out_bf16 as
+ * there, g BF16 [v][h][w][64] = coef (f - target) and partial[b] (b < svbrdf_desc_conv1_loss_partials)
+ * = a block's share of sum (f - target)^2, with f the FP32 features and target FP32 like them; what
+ * svbrdf_desc_feat_loss writes without gram_grad and mask. 16-byte aligned maps. */
+long long svbrdf_desc_conv1_loss_partials(int v, int h, int w);
+int svbrdf_desc_conv1_loss(const float* renders, const float* weight, const float* bias, void* out_bf16, int v, int h,
+                           int w, int downsample, const float* target, float coef, void* g, float* partial,
+                           void* stream);
+
 /* Data gradient of svbrdf_desc_conv1_fwd before its ReLU: gz BF16 NHWC [v][h][w][64] (the
  * masked gradient at conv1_1's output) -> grad_renders FP32 [v][3][2h][2w] (or [v][3][h][w]
  * without `downsample`), overwritten. */
@@ -307,9 +316,9 @@ int svbrdf_desc_avgpool_bwd(const void* gy, const void* x, const void* addend, v
 
 /* Feature term of one hook: partial[b] (b < svbrdf_desc_partials(), if partial) = block b's
  * share of sum (f - t)^2, a fixed-order split; if g: g = coef (f - t) + gram_grad (nullable),
- * times (f > 0) if `mask`, stored BF16. f is BF16 (f_is_bf16) or FP32, t and gram_grad FP32,
- * all n elements. */
-int svbrdf_desc_feat_loss(const void* f, int f_is_bf16, const float* t, const float* gram_grad, float coef, int mask,
+ * times (f > 0) if `mask`, stored BF16. `dtypes` bit 0: f is BF16, else FP32; bit 1: t is BF16,
+ * else FP32; gram_grad FP32; all n elements. */
+int svbrdf_desc_feat_loss(const void* f, int dtypes, const void* t, const float* gram_grad, float coef, int mask,
                           void* g, float* partial, long long n, void* stream);
 
 /* ---- descriptor loss: the Gram term on the tensor cores (the reference's Gram branch

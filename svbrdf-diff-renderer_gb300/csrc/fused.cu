@@ -365,15 +365,16 @@ __device__ __forceinline__ bool run_finish(const char* plan, const PlanHeader* h
   for (int e = w; e < nr * nq; e += NCW + 1) {
     const int r = e / nq, q = e % nq, tile = run_tile[r0 + r];
     const size_t slot = (size_t)tile * NCW + lane;
-    double v = 0.0;
+    float v = 0.0f;  // FP32 here: 16 terms, and double-precision instructions are scarce on this part
     if (lane < NCW) {
-      if (r == nr - 1) v = rows[lane].v[q];
-      else if (lpart && q > 0) v = (double)__ldcg(lpart + 3 * slot + q - 1);
-      else v = (double)__ldcg(partial + (size_t)q * slots + slot);
+      if (r == nr - 1) v = (float)rows[lane].v[q];
+      else if (lpart && q > 0) v = __ldcg(lpart + 3 * slot + q - 1);
+      else v = __ldcg(partial + (size_t)q * slots + slot);
     }
-    v = warp_sum(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) {
-      totals[(size_t)(lpart && q > 0 ? kFuseMax + q - 1 : q) * n_tiles + tile] = (float)v;
+      totals[(size_t)(lpart && q > 0 ? kFuseMax + q - 1 : q) * n_tiles + tile] = v;
       __threadfence();
     }
   }

@@ -180,21 +180,36 @@ class VGGDescriptor:
         return {k: (v["w32"].cpu(), v["b"].cpu()) for k, v in self.params.items()}
 
     # ---- forward -----------------------------------------------------------------------
-    def _forward(self, renders: torch.Tensor):
+    def _forward(self, renders: torch.Tensor, cf: Optional[float] = None):
         """Run the stack. Returns (acts, hooks): acts[i] is the output of layer i of
         self.layers (NHWC BF16); hooks maps each hooked layer to its feature (relu1_1 in
-        FP32, the others BF16)."""
+        FP32, the others BF16). With ``cf`` (no Gram term, targets loaded) relu1_1's feature term
+        runs in the kernel that computes it, and its hook is that term's (gradient, number of
+        partial sums, the buffer of all hooks' partial sums that starts with them) instead of
+        the FP32 feature."""
         L = N.lib()
         st = N.stream_handle(self.device)
         x = renders.detach().float().contiguous()
         v, _, rh, rw = x.shape
         h, w = (rh // 2, rw // 2) if self.downsample else (rh, rw)
         p = self.params["conv1_1"]
-        y32 = torch.empty(v, h, w, 64, device=self.device, dtype=torch.float32)
         y16 = torch.empty(v, h, w, 64, device=self.device, dtype=torch.bfloat16)
-        N.check(L.svbrdf_desc_conv1_fwd(x.data_ptr(), p["w32"].data_ptr(), p["b"].data_ptr(), y32.data_ptr(),
-                                        y16.data_ptr(), v, h, w, int(self.downsample), st))
-        acts, hooks = [y16], {"conv1_1": y32}
+        if cf is not None:
+            t32 = self.target[0][0]
+            if tuple(t32.shape) != (v, h, w, 64):
+                raise ValueError(f"renders give {(v, h, w, 64)} features, the loaded targets {tuple(t32.shape)}")
+            n0 = int(L.svbrdf_desc_conv1_loss_partials(v, h, w))
+            buf = torch.empty(n0 + (len(self.hooks) - 1) * L.svbrdf_desc_partials(), device=self.device,
+                              dtype=torch.float32)
+            hook = (torch.empty_like(y16), n0, buf)
+            N.check(L.svbrdf_desc_conv1_loss(x.data_ptr(), p["w32"].data_ptr(), p["b"].data_ptr(), y16.data_ptr(), v, h,
+                                             w, int(self.downsample), t32.data_ptr(), self._feature_coef(0, cf),
+                                             hook[0].data_ptr(), buf.data_ptr(), st))
+        else:
+            hook = torch.empty(v, h, w, 64, device=self.device, dtype=torch.float32)
+            N.check(L.svbrdf_desc_conv1_fwd(x.data_ptr(), p["w32"].data_ptr(), p["b"].data_ptr(), hook.data_ptr(),
+                                            y16.data_ptr(), v, h, w, int(self.downsample), st))
+        acts, hooks = [y16], {"conv1_1": hook}
         pool_fwd = L.svbrdf_desc_avgpool_fwd if self.avg_pool else L.svbrdf_desc_pool_fwd
         for item in self.layers[1:]:
             prev = acts[-1]
@@ -213,6 +228,11 @@ class VGGDescriptor:
         return acts, hooks
 
     # ---- loss terms --------------------------------------------------------------------
+    def _feature_coef(self, k: int, cf: float) -> float:
+        """cf d(feature loss)/d(f - t) of hook k, per unit of f - t: 2 w_k^2 / (all hooks' elements)."""
+        wt = self.hook_weights[k]
+        return 2.0 * wt * wt * cf / sum(t.numel() for t in self.target[0])
+
     def _terms(self, hooks, cf: Optional[float], cg: Optional[float], hooks16=None):
         """Feature and Gram losses (0-d FP32 tensors). With cf/cg given, also the loss
         gradient at each hooked activation, cf d(feature)/df + cg d(gram)/df, as BF16 NHWC; the
@@ -222,34 +242,40 @@ class VGGDescriptor:
         L = N.lib()
         st = N.stream_handle(self.device)
         tf, tg = self.target
+        # relu1_1's term where the forward pass has run it: (gradient, partial sums, all hooks' buffer)
+        done = hooks["conv1_1"] if isinstance(hooks["conv1_1"], tuple) else None
         if hooks16 is None:
             hooks16 = {n: (f if f.dtype == torch.bfloat16 else f.to(torch.bfloat16)) for n, f in hooks.items()}
-        nf = sum(f.numel() for f in hooks.values())
+        nf = sum(t.numel() for t in tf)
         ng = sum(g.numel() for g in tg)
         nparts = L.svbrdf_desc_partials()
         fused = cf is not None and self.gram
         # segments: each hook's feature partials, then each hook's Gram loss rows
         lens, weights, groups = [], [], []
-        for name, wt in zip(self.hooks, self.hook_weights):
-            v, h, w, c = hooks[name].shape
-            lens.append(int(L.svbrdf_desc_gemm_nt_feat_partials(v, h * w, c)) if fused else nparts)
+        for name, wt, t in zip(self.hooks, self.hook_weights, tf):
+            v, h, w, c = t.shape
+            lens.append(int(L.svbrdf_desc_gemm_nt_feat_partials(v, h * w, c)) if fused else
+                        done[1] if done and name == "conv1_1" else nparts)
             weights.append(wt * wt / nf)
             groups.append(0)
         if self.gram:
-            for name, wt in zip(self.hooks, self.hook_weights):
-                v, h, w, c = hooks[name].shape
+            for name, wt, t in zip(self.hooks, self.hook_weights, tf):
+                v, h, w, c = t.shape
                 lens.append(v * c)
                 weights.append(wt * wt / ng)
                 groups.append(1)
         offs = [0]
         for n in lens[:-1]:
             offs.append(offs[-1] + n)
-        buf = torch.empty(offs[-1] + lens[-1], device=self.device, dtype=torch.float32)
+        buf = done[2] if done else torch.empty(offs[-1] + lens[-1], device=self.device, dtype=torch.float32)
         nh = len(self.hooks)
         grads = {}
         last = [it for it in self.layers if it != "pool"][-1][0]
         for k, (name, wt) in enumerate(zip(self.hooks, self.hook_weights)):
             f = hooks[name]
+            if done and name == "conv1_1":
+                grads[name] = done[0]
+                continue
             v, h, w, c = f.shape
             s = h * w
             part = buf[offs[k]:offs[k] + lens[k]]
@@ -265,19 +291,19 @@ class VGGDescriptor:
             if cf is not None:
                 g = torch.empty(v, h, w, c, device=self.device, dtype=torch.bfloat16)
                 grads[name] = g
+            # a BF16 hook's targets are read in BF16 (exact: they are BF16 values)
+            t16 = self.target16[k] if getattr(self, "target16", None) else None
+            dtypes = int(f.dtype == torch.bfloat16) | (2 if t16 is not None else 0)
+            t = t16 if t16 is not None else tf[k]
             if fused:
-                # the Gram gradient F dG with this hook's feature term in its epilogue; a BF16
-                # hook's targets are read in BF16 (exact: they are BF16 values)
-                t16 = self.target16[k] if getattr(self, "target16", None) else None
-                dtypes = int(f.dtype == torch.bfloat16) | (2 if t16 is not None else 0)
+                # the Gram gradient F dG with this hook's feature term in its epilogue
                 N.check(L.svbrdf_desc_gemm_nt_feat(ff.data_ptr(), dgram.data_ptr(), f.data_ptr(), dtypes,
-                                                   (t16 if t16 is not None else tf[k]).data_ptr(), coef,
+                                                   t.data_ptr(), coef,
                                                    int(name == last), g.data_ptr(), part.data_ptr(), v, s, c, c,
                                                    self.err.data_ptr(), st))
             else:
-                N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), int(f.dtype == torch.bfloat16), tf[k].data_ptr(),
-                                                None, coef, int(name == last), N.ptr(g), part.data_ptr(),
-                                                f.numel(), st))
+                N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), dtypes, t.data_ptr(), None, coef,
+                                                int(name == last), N.ptr(g), part.data_ptr(), f.numel(), st))
         out = torch.empty(2, device=self.device, dtype=torch.float32)
         ns = len(lens)
         a_off = (ctypes.c_longlong * ns)(*offs)
@@ -389,7 +415,7 @@ class VGGDescriptor:
         self._graph = (tuple(shape), graph, static_r, fl, gl, dr)
 
     def _loss_and_grad_eager(self, renders):
-        acts, hooks = self._forward(renders)
+        acts, hooks = self._forward(renders, None if self.gram else 1.0)
         fl, gl, grads = self._terms(hooks, 1.0, 1.0, self._bf16_hooks(acts, hooks))
         return fl, gl, self._backward(acts, grads, renders.shape)
 

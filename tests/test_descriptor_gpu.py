@@ -450,3 +450,75 @@ def test_descriptor_at_config_shape_vs_fp64_oracle(svb, cuda):
     e_q, e_r = rel_l2(g0, q0), rel_l2(g0, r0)
     print(f"9 x 512^2, view 0: d/drender vs BF16-activation FP64 {e_q:.2e}, vs FP64 {e_r:.2e}")
     assert e_q <= 0.1 and e_r <= 0.3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 16, 16), (2, 48, 80), (3, 64, 32), (1, 8, 20), (2, 100, 9)])
+@pytest.mark.parametrize("down", [0, 1])
+def test_conv1_loss_equals_its_two_kernels(svb, cuda, shape, down):
+    """conv1_1 with its hook's feature term in one kernel against the convolution and the feature-loss
+    kernel, on whole and clipped tiles and one to several tile rows per block: the BF16 outputs equal,
+    the squared sum (FP32, another order over at most 64 x 6400 terms) within 1e-5."""
+    v, h, w = shape
+    N, L = svb._native, svb._native.lib()
+    g = torch.Generator(device=cuda).manual_seed(h * w)
+    r = torch.rand(v, 3, h * (1 + down), w * (1 + down), generator=g, device=cuda)
+    wt, b = torch.randn(64, 3, 3, 3, generator=g, device=cuda) * 0.3, torch.randn(64, generator=g, device=cuda) * 0.1
+    t = torch.rand(v, h, w, 64, generator=g, device=cuda)
+    st = N.stream_handle(cuda)
+    y32, y16, y16b = (torch.empty(v, h, w, 64, device=cuda, dtype=d) for d in (torch.float32, torch.bfloat16, torch.bfloat16))
+    ga, gb = torch.empty_like(y16), torch.empty_like(y16)
+    pa = torch.zeros(L.svbrdf_desc_partials(), device=cuda)
+    pb = torch.zeros(L.svbrdf_desc_conv1_loss_partials(v, h, w), device=cuda)
+    N.check(L.svbrdf_desc_conv1_fwd(r.data_ptr(), wt.data_ptr(), b.data_ptr(), y32.data_ptr(), y16.data_ptr(), v, h, w,
+                                    down, st))
+    N.check(L.svbrdf_desc_feat_loss(y32.data_ptr(), 0, t.data_ptr(), None, 0.37, 0, ga.data_ptr(), pa.data_ptr(),
+                                    y32.numel(), st))
+    N.check(L.svbrdf_desc_conv1_loss(r.data_ptr(), wt.data_ptr(), b.data_ptr(), y16b.data_ptr(), v, h, w, down,
+                                     t.data_ptr(), 0.37, gb.data_ptr(), pb.data_ptr(), st))
+    assert torch.equal(y16, y16b) and torch.equal(ga, gb)
+    assert torch.equal(y32.to(torch.bfloat16), y16)
+    a, c = pa.double().sum(), pb.double().sum()
+    assert abs(float(a - c)) <= 1e-5 * float(a)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 7, 8, 1000, 2 ** 21 + 8, 2 ** 22 + 4])
+@pytest.mark.parametrize("dtypes", [0, 1, 2, 3])
+def test_feature_loss_types_and_sizes(svb, cuda, n, dtypes):
+    """The feature term in 16-byte vectors (n a multiple of 8) and one element at a time, FP32 and
+    BF16 features and targets, with the mask and a Gram gradient, against FP64: the BF16 gradient
+    within one BF16 rounding (2^-8), the squared sum within 1e-5."""
+    N, L = svb._native, svb._native.lib()
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    bf = lambda t, on: t.to(torch.bfloat16) if on else t
+    f = bf(torch.randn(n, generator=gen, device=cuda), dtypes & 1)
+    t = bf(torch.randn(n, generator=gen, device=cuda), dtypes & 2)
+    gg = torch.randn(n, generator=gen, device=cuda)
+    g, p = torch.empty(n, device=cuda, dtype=torch.bfloat16), torch.zeros(L.svbrdf_desc_partials(), device=cuda)
+    N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), dtypes, t.data_ptr(), gg.data_ptr(), 0.7, 1, g.data_ptr(),
+                                    p.data_ptr(), n, N.stream_handle(cuda)))
+    d = f.double() - t.double()
+    want = torch.where(f > 0, 0.7 * d + gg.double(), torch.zeros_like(d))
+    assert ((g.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6).all()
+    assert abs(float(p.double().sum() - (d * d).sum())) <= 1e-5 * float((d * d).sum())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[1], [300, 0, 5], [9000, 255, 256, 257, 18432], [31] * 16])
+def test_loss_sums_segments(svb, cuda, lens):
+    """The weighted sums of two groups over segments shorter and longer than the 256 floats of a
+    unit, empty ones and the most there can be, against FP64 (sums of positive FP32 terms: 1e-6)."""
+    import ctypes
+    N, L = svb._native, svb._native.lib()
+    buf = torch.rand(sum(lens) + 1, device=cuda, generator=torch.Generator(device=cuda).manual_seed(len(lens)))
+    offs = [sum(lens[:k]) for k in range(len(lens))]
+    w, grp = [0.5 + 0.1 * k for k in range(len(lens))], [k % 2 for k in range(len(lens))]
+    out = torch.empty(2, device=cuda)
+    n = len(lens)
+    arr = [(ctypes.c_longlong * n)(*offs), (ctypes.c_longlong * n)(*lens), (ctypes.c_double * n)(*w), (ctypes.c_int * n)(*grp)]
+    N.check(L.svbrdf_desc_loss_sums(buf.data_ptr(), n, *[ctypes.addressof(a) for a in arr], out.data_ptr(),
+                                    N.stream_handle(cuda)))
+    for j in range(2):
+        want = sum(w[k] * float(buf[offs[k]:offs[k] + lens[k]].double().sum()) for k in range(n) if grp[k] == j)
+        assert abs(float(out[j]) - want) <= 1e-6 * max(want, 1e-30)
