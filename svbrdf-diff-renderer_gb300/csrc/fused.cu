@@ -373,19 +373,18 @@ __device__ __forceinline__ bool run_finish(const char* plan, const PlanHeader* h
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) {
-      totals[(size_t)(lpart && q > 0 ? kFuseMax + q - 1 : q) * n_tiles + tile] = v;
-      __threadfence();
-    }
+    if (lane == 0) totals[(size_t)(lpart && q > 0 ? kFuseMax + q - 1 : q) * n_tiles + tile] = v;
   }
+  // one thread's fences order the whole block's accesses, which the barriers put before and after them
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    *s_flag = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1 : 0;
+    const int last = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1 : 0;
+    if (last) __threadfence();
+    *s_flag = last;
   }
   __syncthreads();
   if (!*s_flag) return false;
-  __threadfence();
   // one warp per (material, quantity)
   for (int e = w; e < hdr->n_mat * nq; e += NCW + 1) {
     const int mi = e / nq, q = e % nq;
@@ -425,7 +424,6 @@ __device__ __forceinline__ bool batched_next_iteration(bool last, unsigned* ws, 
   if (threadIdx.x == 0) {
     int ok = 1;
     if (last) {
-      __threadfence();
       asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ws + kWsIteration), "r"(number) : "memory");
     } else {
       for (uint32_t it = 0;; ++it) {
@@ -438,7 +436,6 @@ __device__ __forceinline__ bool batched_next_iteration(bool last, unsigned* ws, 
           break;
         }
       }
-      __threadfence();
     }
     *s_flag = ok;
   }
@@ -973,6 +970,9 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   long long issued = 0;
   bool ok = true;
   RingCursor rc{0, 0u, true};
+  const int4* seq = (const int4*)(plan + hdr->off_seq);
+  const int4 sq_first = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
+  int cur = -1;  // the producer's staged material
 
   for (int it = 0; it < iters; ++it) {
     if (warp == NCW) {
@@ -981,21 +981,25 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       // release that publishes the record); lanes 0 .. nplanes-1 then issue one plane copy
       // each. The next tile's entry is loaded one tile ahead and a material's fields and
       // views only when the material changes.
-      const int4* seq = (const int4*)(plan + hdr->off_seq);
       const bool was_ok = ok;
-      int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
-      int cur = -1, run_tile = 0;
+      int4 sq_next = sq_first;
+      int run_tile = 0;
       for (int k = k0; k < k1 && ok; ++k) {
         const int4 sq = sq_next;
         if (k + 1 < n_tiles) sq_next = seq[k + 1];
-        if (sq.y != cur) {
+        if (sq.y != cur || k == k0) {
+          // the material's fields and views are staged still if the last iteration ended with it;
+          // its light power may have been stepped since, by another CTA
+          const bool staged = sq.y == cur;
           cur = sq.y;
           run_tile = sq.x;
           __syncwarp();
           const MatDesc& m = mats[cur];
-          if (lane == 0) s_prod_md = m;
-          if (lane < 3) s_prod_pow[lane] = __ldcg(m.lpow + lane);  // another CTA may have stepped it
-          for (int v = lane; v < m.V; v += 32) s_prod_views[v] = views[m.view_off + v];
+          if (!staged) {
+            if (lane == 0) s_prod_md = m;
+            for (int v = lane; v < m.V; v += 32) s_prod_views[v] = views[m.view_off + v];
+          }
+          if (lane < 3) s_prod_pow[lane] = __ldcg((staged ? s_prod_md.lpow : m.lpow) + lane);
           __syncwarp();
         }
         const MatDesc& md = s_prod_md;
