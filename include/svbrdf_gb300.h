@@ -288,9 +288,9 @@ int svbrdf_desc_conv1_loss(const float* renders, const float* weight, const floa
 int svbrdf_desc_conv1_bwd(const void* gz, const float* weight, float* grad_renders, int v, int h, int w,
                           int downsample, void* stream);
 
-/* The same data gradient on the tensor cores: the 64 -> 3 channel 3x3 convolution as a BF16
- * tcgen05 implicit GEMM (N = 16: weight rows 3..15 zero), FP32 accumulation. w16: BF16
- * [16][9][64], row c, tap 3 ky + kx, channel k = conv1_1's weight[k][c][2 - ky][2 - kx] for
+/* The same data gradient on the tensor cores: the 9 taps x 3 channels as the columns of one BF16
+ * tcgen05 product per pixel row, FP32 accumulation, the shifted results added in FP32. w16: BF16
+ * [16][9][64] (rows 3..15 unused), row c, tap 3 ky + kx, channel k = conv1_1's weight[k][c][2 - ky][2 - kx] for
  * c < 3. scale[c] (FP32, 3 values) multiplies channel c: 1 / std[c] of the normalisation, times
  * 1/4 with `downsample` (the box filter's adjoint gives each of the window's 4 render pixels
  * the scaled value). h % 8 == 0, w % 16 == 0; gz and w16 16-byte aligned, grad_renders

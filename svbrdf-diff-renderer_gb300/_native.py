@@ -22,7 +22,7 @@ CSRC = PKG / "csrc"
 INCLUDE = REPO / "include"
 LIBDIR = PKG / "_lib"
 LIBNAME = "libsvbrdf_gb300.so"
-SOURCES = ["render.cu", "fused.cu", "conv_tc.cu", "gram_tc.cu", "conv_tf32.cu", "desc_ops.cu", "gen_ops.cu",
+SOURCES = ["render.cu", "fused.cu", "conv_tc.cu", "conv1_grad_tc.cu", "gram_tc.cu", "conv_tf32.cu", "desc_ops.cu", "gen_ops.cu",
            "gen_nhwc.cu", "envmap.cu"]
 HEADERS = ["svbrdf_math.cuh", "svbrdf_common.cuh", "svbrdf_plan.cuh", "tc_ptx.cuh"]
 WORKSPACE_ERROR_OFFSET = 4

@@ -44,13 +44,8 @@ constexpr int kEpiWarps = 8;  // two per TMEM lane quadrant, each draining half 
 // output; the epilogue routes it back to the pool's input (the window's first maximum, or a
 // quarter to each element), adds the addend there and applies the ReLU mask of the pool's input.
 // `mask` is the pool's input and `y` the gradient at it, both [N, 2H, 2W, Cout].
-// kEpiRenderDown / kEpiRender (BN = 16, the data gradient of the descriptor's first layer,
-// 64 -> 3 channels padded to 16): channel c < 3 of the accumulator times scale[c] (`bias`) is the
-// gradient at the normalised render, written FP32 NCHW to `y` [N][3][2H][2W] through the 2x2
-// box downsample's adjoint (each of the window's 4 pixels takes the value; the 1/4 is in scale)
-// or [N][3][H][W] without it.
 enum Epilogue : int { kEpiNone = 0, kEpiBiasRelu = 1, kEpiMask = 2, kEpiAddMask = 3, kEpiUnpoolMax = 4,
-                      kEpiUnpoolAvg = 5, kEpiRenderDown = 6, kEpiRender = 7 };
+                      kEpiUnpoolAvg = 5 };
 enum ConvError : int { kErrTma = 11, kErrMma = 12, kErrEpi = 13 };
 
 // One accumulator row (an output pixel) of 32 channels through the epilogue, stored as BF16;
@@ -395,8 +390,8 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // values of the first PF chunks depend only on the tile's coordinates, so they are loaded
     // before the wait for the accumulator.
     constexpr bool BYTILE = BN == 64 && MT == 2;
-    constexpr int CPH = BYTILE ? 2 : (BN >= 64 ? BN / 64 : 1);  // 32-column chunks per M-tile drained
-    constexpr int NCH = BN >= 64 ? (BYTILE ? 1 : MT) * CPH : 0;  // BN = 16 (the render epilogues) drains below
+    constexpr int CPH = BYTILE ? 2 : BN / 64;  // 32-column chunks per M-tile drained
+    constexpr int NCH = (BYTILE ? 1 : MT) * CPH;
     constexpr int PF = EPI == kEpiMask ? (NCH < 4 ? NCH : 4) : EPI == kEpiAddMask ? (NCH < 2 ? NCH : 2) : 0;
     const int qw = warp & 3;        // the TMEM lane quadrant this warp may read
     const int half = (warp - 2) >> 2;  // which half of the columns (or which M-tile) it drains
@@ -473,29 +468,6 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         if (lane == 0) {
           tma_store_4d(&tmap_y, sbase + (uint32_t)((warp - 2) * 4096), n0, x0, y0 + 16 * mt0 + 4 * qw, img);
           bulk_commit();
-        }
-      }
-      if ((EPI == kEpiRenderDown || EPI == kEpiRender) && half == 0) {
-        float* dr = reinterpret_cast<float*>(y);
-        const int px = x0 + m % 8;
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int py = y0 + 16 * mt + m / 8;
-          uint32_t r[4];
-          tmem_ld4(tmem + ((uint32_t)(qw * 32) << 16) + (uint32_t)(a * ACC_COLS + mt * BN), r);
-          if (py < H) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const float val = __uint_as_float(r[c]) * __ldg(bias + c);
-              if (EPI == kEpiRenderDown) {
-                float* row = dr + (((size_t)img * 3 + c) * 2 * H + 2 * py) * (size_t)(2 * W) + 2 * px;
-                *reinterpret_cast<float2*>(row) = make_float2(val, val);
-                *reinterpret_cast<float2*>(row + 2 * W) = make_float2(val, val);
-              } else {
-                dr[(((size_t)img * 3 + c) * H + py) * (size_t)W + px] = val;
-              }
-            }
-          }
         }
       }
       fence_before();
@@ -697,50 +669,6 @@ extern "C" int svbrdf_conv3x3_bf16_ex(const void* x, const void* weight, const f
                        : dispatch_halo<64, 1>(epilogue, mh, mw, pmy, bias, mask, addend, y, n, h, w, cin, cout, err, st);
     }
   }
-}
-
-extern "C" int svbrdf_desc_conv1_bwd_tc(const void* gz, const void* w16, const float* scale, float* dr, int n, int h,
-                                        int w, int down, int* err, void* stream) {
-  using namespace svb::tc;
-  if (!gz || !w16 || !scale || !dr || !err) return fail(SVBRDF_ERR_INVALID, "conv1_bwd_tc: null argument");
-  if (n < 1 || n > 65535 || h < TH || w < TW || h % TH || w % TW)
-    return fail(SVBRDF_ERR_UNSUPPORTED, "conv1_bwd_tc: H must be a multiple of %d and W of %d (got %dx%d)", TH, TW, h,
-                w);
-  if (((uintptr_t)gz | (uintptr_t)w16) % 16 || (uintptr_t)dr % 8)
-    return fail(SVBRDF_ERR_INVALID, "conv1_bwd_tc: gz / w16 must be 16-byte aligned, dr 8-byte aligned");
-  if ((long long)n * h * w * 64 >= (1LL << 40)) return fail(SVBRDF_ERR_UNSUPPORTED, "conv1_bwd_tc: tensor too large");
-  PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-  int rc = get_tensor_map_encoder(&g_encode);
-  if (rc) return rc;
-  CUtensorMap mw, mh;
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)9 * 64, 16};
-    const cuuint64_t strides[1] = {(cuuint64_t)9 * 64 * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, 16u};
-    const cuuint32_t es[2] = {1, 1};
-    const CUresult r = g_encode(&mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w16), dims, strides, box,
-                                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(SVBRDF_ERR_CUDA, "cuTensorMapEncodeTiled(w16) failed: %d", (int)r);
-  }
-  const int mt = h >= 32 ? 2 : 1;
-  {
-    const cuuint64_t dims[4] = {64, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    const cuuint64_t strides[3] = {64 * 2, (cuuint64_t)w * 64 * 2, (cuuint64_t)h * w * 64 * 2};
-    const cuuint32_t box[4] = {(cuuint32_t)BK, 10u, (cuuint32_t)(16 * mt + 2), 1u};
-    const cuuint32_t es[4] = {1, 1, 1, 1};
-    const CUresult r = g_encode(&mh, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(gz), dims, strides, box,
-                                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(SVBRDF_ERR_CUDA, "cuTensorMapEncodeTiled(gz) failed: %d", (int)r);
-  }
-  cudaStream_t st = (cudaStream_t)stream;
-  void* y = dr;
-  if (down)
-    return mt == 2 ? launch_halo<16, 2, kEpiRenderDown>(mh, mw, nullptr, scale, nullptr, nullptr, y, n, h, w, 64, 16, err, st)
-                   : launch_halo<16, 1, kEpiRenderDown>(mh, mw, nullptr, scale, nullptr, nullptr, y, n, h, w, 64, 16, err, st);
-  return mt == 2 ? launch_halo<16, 2, kEpiRender>(mh, mw, nullptr, scale, nullptr, nullptr, y, n, h, w, 64, 16, err, st)
-                 : launch_halo<16, 1, kEpiRender>(mh, mw, nullptr, scale, nullptr, nullptr, y, n, h, w, 64, 16, err, st);
 }
 
 extern "C" int svbrdf_conv3x3_bf16(const void* x, const void* weight, const float* bias, const void* mask, void* y,

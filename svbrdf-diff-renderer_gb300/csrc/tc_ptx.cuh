@@ -1,4 +1,4 @@
-// Inline-PTX helpers of the tcgen05 kernels (conv_tc.cu, gram_tc.cu): mbarriers with bounded
+// Inline-PTX helpers of the tcgen05 kernels (conv_tc.cu, conv1_grad_tc.cu, gram_tc.cu): mbarriers with bounded
 // waits, TMA tensor loads, shared-memory matrix descriptors, tcgen05.mma / commit / ld, and the
 // tensor-map encoder looked up from the driver.
 #pragma once
@@ -123,14 +123,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Columns 0..3 of this warp's 32 TMEM lanes starting at `taddr`.
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 

@@ -522,3 +522,28 @@ def test_loss_sums_segments(svb, cuda, lens):
     for j in range(2):
         want = sum(w[k] * float(buf[offs[k]:offs[k] + lens[k]].double().sum()) for k in range(n) if grp[k] == j)
         assert abs(float(out[j]) - want) <= 1e-6 * max(want, 1e-30)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("v,h,w", [(1, 8, 16), (2, 16, 112), (1, 24, 128), (1, 8, 144), (9, 128, 256), (2, 16, 272),
+                                   (1, 32, 512), (40, 64, 64)])
+@pytest.mark.parametrize("down", [0, 1])
+def test_conv1_bwd_tc_widths_and_strips(svb, cuda, v, h, w, down):
+    """conv1_1's data gradient on maps of one and two 128-pixel tiles and of overlapping windows,
+    full and partly filled, and strips of 4 rows to a whole map, against torch in FP64 on the CPU (the
+    BF16 products are exact in FP32, sums of 576: relative L2 within 1e-5)."""
+    N, L = svb._native, svb._native.lib()
+    p = svb.descriptor.VGGDescriptor(cuda, seed=9, downsample=bool(down)).params["conv1_1"]
+    gz = torch.randn(v, h, w, 64, generator=torch.Generator().manual_seed(h + w)).to(torch.bfloat16)
+    dr = torch.full((v, 3, h * (1 + down), w * (1 + down)), float("nan"), device=cuda)
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    gd = gz.to(cuda)
+    N.check(L.svbrdf_desc_conv1_bwd_tc(gd.data_ptr(), p["w_dg16"].data_ptr(), p["dg_scale"].data_ptr(), dr.data_ptr(), v,
+                                       h, w, down, err.data_ptr(), N.stream_handle(cuda)))
+    assert int(err.item()) == 0
+    gn = torch.nn.functional.conv_transpose2d(gz.double().permute(0, 3, 1, 2), p["w32"].cpu().double(), padding=1)
+    gn = gn / torch.tensor(svb.descriptor.STD, dtype=torch.float64).view(1, 3, 1, 1)
+    want = (0.25 * gn).repeat_interleave(2, 2).repeat_interleave(2, 3) if down else gn
+    assert not torch.isnan(dr).any()
+    assert rel_l2(dr, want) <= 1e-5
+    assert float((dr.cpu().double() - want).abs().max()) <= 1e-4 * float(want.abs().max())
