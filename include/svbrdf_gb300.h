@@ -314,6 +314,14 @@ int svbrdf_desc_avgpool_fwd(const void* x, void* y, int v, int h, int w, int c, 
 int svbrdf_desc_avgpool_bwd(const void* gy, const void* x, const void* addend, void* gx, int v, int h, int w, int c,
                             void* stream);
 
+/* The backward pass of the pool (average with `avg`, else max) with the hook gradient made in place:
+ * addend = coef (x - target) rounded to BF16, target BF16 like x, and partial[b]
+ * (b < svbrdf_desc_pool_bwd_loss_partials) = a block's share of sum (x - target)^2; what
+ * svbrdf_desc_feat_loss (dtypes 3, no gram_grad, no mask) writes, without its pass. */
+long long svbrdf_desc_pool_bwd_loss_partials(int v, int h, int w, int c);
+int svbrdf_desc_pool_bwd_loss(const void* gy, const void* x, const void* target, float coef, void* gx, float* partial,
+                              int v, int h, int w, int c, int avg, void* stream);
+
 /* Feature term of one hook: partial[b] (b < svbrdf_desc_partials(), if partial) = block b's
  * share of sum (f - t)^2, a fixed-order split; if g: g = coef (f - t) + gram_grad (nullable),
  * times (f > 0) if `mask`, stored BF16. `dtypes` bit 0: f is BF16, else FP32; bit 1: t is BF16,

@@ -10,7 +10,7 @@
 //   desc_pool_fwd_kernel   2x2 max-pool (or average pool), NHWC BF16
 //   desc_pool_bwd_kernel   its backward (max: the first maximum of each window takes the
 //                          gradient, as ATen's pool; average: a quarter to each) + optional
-//                          hook gradient + ReLU mask
+//                          hook gradient (given, or made from the hook's feature term) + ReLU mask
 //   desc_feat_loss_kernel  sum of (f - t)^2 as per-block partials (a fixed-order sum), and
 //                          optionally g = coef (f - t) + gram_grad, masked by f > 0
 //   desc_loss_sums_kernel  weighted sums of loss partials (fixed order)
@@ -333,18 +333,23 @@ __global__ void desc_pool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_b
 // gradient. AVG: every element of the window takes gy / 4. Each thread issues all of its loads
 // (the window's x, gy, the window's addend: nine 16-byte loads) before any arithmetic, keeping
 // them as raw BF16 until use.
+// LOSS: the addend is not read but made here, where the hook's feature x is read anyway, as
+// desc_feat_loss_kernel computes it: d = x - t with t the BF16 target that `addend` points to, coef d
+// rounded to BF16, partial[block] = sum d^2. The hook's term then takes no pass of its own (9 maps of
+// 256^2 x 64, relu1_2: 43 + 37 -> 43 us, HBM-bound as both were).
 __device__ __forceinline__ float2 bf2f(const uint4& u, int e) {
   return __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&u)[e]);
 }
-template <bool AVG>
+template <bool AVG, bool LOSS>
 __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16* __restrict__ gy,
                                                             const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ addend,
                                                             __nv_bfloat16* __restrict__ gx, int V, int H, int W,
-                                                            int C) {
+                                                            int C, float coef, float* __restrict__ partial) {
   // grid (ceil(Wo C8 / 256), V Ho): block row (v, yo); thread t of the row is (xo, c8)
   const int Ho = H / 2, Wo = W / 2, C8 = C / 8;
   const int v = blockIdx.y / Ho, yo = blockIdx.y % Ho;
+  float sq = 0.0f;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < Wo * C8; t += gridDim.x * blockDim.x) {
     const int c8 = t % C8, xo = t / C8;
     const size_t p = ((size_t)v * Ho + yo) * Wo + xo;
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
 #pragma unroll
     for (int k = 0; k < 4; ++k) xr[k] = __ldg(reinterpret_cast<const uint4*>(x + b0 + offs[k]));
     const uint4 gr = __ldg(reinterpret_cast<const uint4*>(gy + p * C + c8 * 8));
-    if (addend) {
+    if (LOSS || addend) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) ar[k] = __ldg(reinterpret_cast<const uint4*>(addend + b0 + offs[k]));
     } else {
@@ -379,7 +384,13 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float2 ad = bf2f(ar[k], e);
+        float2 ad = bf2f(ar[k], e);
+        if constexpr (LOSS) {
+          const float2 d = make_float2(xv[k].x - ad.x, xv[k].y - ad.y);
+          sq = fmaf(d.x, d.x, sq);
+          sq = fmaf(d.y, d.y, sq);
+          ad = __bfloat1622float2(__floats2bfloat162_rn(coef * d.x, coef * d.y));
+        }
         float vx = AVG ? 0.25f * g.x : (amx == k ? g.x : 0.0f);
         float vy = AVG ? 0.25f * g.y : (amy == k ? g.y : 0.0f);
         vx += ad.x;
@@ -390,6 +401,18 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(gx + b0 + offs[k]) = o[k];
+  }
+  if constexpr (LOSS) {
+    __shared__ float s_red[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float s = 0.0f;
+      for (int w = 0; w < 8; ++w) s += s_red[w];
+      partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
+    }
   }
 }
 
@@ -559,6 +582,10 @@ static int conv1_fwd(const float* renders, const float* weight, const float* bia
   return check_launch("desc_conv1_fwd_kernel");
 }
 
+static dim3 pool_grid(int v, int h, int w, int c) {
+  return dim3((unsigned)(((w / 2) * (c / 8) + 255) / 256), (unsigned)(v * (h / 2)));
+}
+
 template <bool AVG>
 static int pool_fwd(const void* x, void* y, int v, int h, int w, int c, void* stream) {
   if (!x || !y) return fail(SVBRDF_ERR_INVALID, "null pointer");
@@ -567,26 +594,24 @@ static int pool_fwd(const void* x, void* y, int v, int h, int w, int c, void* st
   if (((uintptr_t)x | (uintptr_t)y) % 16) return fail(SVBRDF_ERR_INVALID, "pool: 16-byte alignment needed");
   if ((long long)v * (h / 2) > 65535 || (long long)(w / 2) * (c / 8) >= (1LL << 30))
     return fail(SVBRDF_ERR_UNSUPPORTED, "pool: too large");
-  const dim3 grid((unsigned)(((w / 2) * (c / 8) + 255) / 256), (unsigned)(v * (h / 2)));
-  desc_pool_fwd_kernel<AVG><<<grid, 256, 0, (cudaStream_t)stream>>>(
+  desc_pool_fwd_kernel<AVG><<<pool_grid(v, h, w, c), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)x, (__nv_bfloat16*)y, v, h, w, c);
   return check_launch("desc_pool_fwd_kernel");
 }
 
-template <bool AVG>
+template <bool AVG, bool LOSS>
 static int pool_bwd(const void* gy, const void* x, const void* addend, void* gx, int v, int h, int w, int c,
-                    void* stream) {
-  if (!gy || !x || !gx) return fail(SVBRDF_ERR_INVALID, "null pointer");
+                    float coef, float* partial, void* stream) {
+  if (!gy || !x || !gx || (LOSS && (!addend || !partial))) return fail(SVBRDF_ERR_INVALID, "null pointer");
   if (v < 1 || h < 2 || w < 2 || h % 2 || w % 2 || c < 8 || c % 8)
     return fail(SVBRDF_ERR_UNSUPPORTED, "pool: even H, W and C a multiple of 8 needed");
   if (((uintptr_t)gy | (uintptr_t)x | (uintptr_t)addend | (uintptr_t)gx) % 16)
     return fail(SVBRDF_ERR_INVALID, "pool: 16-byte alignment needed");
   if ((long long)v * (h / 2) > 65535 || (long long)(w / 2) * (c / 8) >= (1LL << 30))
     return fail(SVBRDF_ERR_UNSUPPORTED, "pool: too large");
-  const dim3 grid((unsigned)(((w / 2) * (c / 8) + 255) / 256), (unsigned)(v * (h / 2)));
-  desc_pool_bwd_kernel<AVG><<<grid, 256, 0, (cudaStream_t)stream>>>(
+  desc_pool_bwd_kernel<AVG, LOSS><<<pool_grid(v, h, w, c), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)gy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)addend, (__nv_bfloat16*)gx, v, h, w,
-      c);
+      c, coef, partial);
   return check_launch("desc_pool_bwd_kernel");
 }
 
@@ -642,7 +667,7 @@ int svbrdf_desc_pool_fwd(const void* x, void* y, int v, int h, int w, int c, voi
 
 int svbrdf_desc_pool_bwd(const void* gy, const void* x, const void* addend, void* gx, int v, int h, int w, int c,
                          void* stream) {
-  return pool_bwd<false>(gy, x, addend, gx, v, h, w, c, stream);
+  return pool_bwd<false, false>(gy, x, addend, gx, v, h, w, c, 0.0f, nullptr, stream);
 }
 
 int svbrdf_desc_avgpool_fwd(const void* x, void* y, int v, int h, int w, int c, void* stream) {
@@ -651,7 +676,19 @@ int svbrdf_desc_avgpool_fwd(const void* x, void* y, int v, int h, int w, int c, 
 
 int svbrdf_desc_avgpool_bwd(const void* gy, const void* x, const void* addend, void* gx, int v, int h, int w, int c,
                             void* stream) {
-  return pool_bwd<true>(gy, x, addend, gx, v, h, w, c, stream);
+  return pool_bwd<true, false>(gy, x, addend, gx, v, h, w, c, 0.0f, nullptr, stream);
+}
+
+long long svbrdf_desc_pool_bwd_loss_partials(int v, int h, int w, int c) {
+  if (v < 1 || h < 2 || w < 2 || c < 8) return 0;
+  const dim3 g = pool_grid(v, h, w, c);
+  return (long long)g.x * g.y;
+}
+
+int svbrdf_desc_pool_bwd_loss(const void* gy, const void* x, const void* target, float coef, void* gx, float* partial,
+                              int v, int h, int w, int c, int avg, void* stream) {
+  return avg ? pool_bwd<true, true>(gy, x, target, gx, v, h, w, c, coef, partial, stream)
+             : pool_bwd<false, true>(gy, x, target, gx, v, h, w, c, coef, partial, stream);
 }
 
 int svbrdf_desc_feat_loss(const void* f, int dtypes, const void* t, const float* gram_grad, float coef, int mask,

@@ -184,8 +184,8 @@ class VGGDescriptor:
         """Run the stack. Returns (acts, hooks): acts[i] is the output of layer i of
         self.layers (NHWC BF16); hooks maps each hooked layer to its feature (relu1_1 in
         FP32, the others BF16). With ``cf`` (no Gram term, targets loaded) relu1_1's feature term
-        runs in the kernel that computes it, and its hook is that term's (gradient, number of
-        partial sums, the buffer of all hooks' partial sums that starts with them) instead of
+        runs in the kernel that computes it, and its hook is that term's (gradient, every hook's
+        number of partial sums, the buffer of them all that starts with this term's) instead of
         the FP32 feature."""
         L = N.lib()
         st = N.stream_handle(self.device)
@@ -198,10 +198,10 @@ class VGGDescriptor:
             t32 = self.target[0][0]
             if tuple(t32.shape) != (v, h, w, 64):
                 raise ValueError(f"renders give {(v, h, w, 64)} features, the loaded targets {tuple(t32.shape)}")
-            n0 = int(L.svbrdf_desc_conv1_loss_partials(v, h, w))
-            buf = torch.empty(n0 + (len(self.hooks) - 1) * L.svbrdf_desc_partials(), device=self.device,
-                              dtype=torch.float32)
-            hook = (torch.empty_like(y16), n0, buf)
+            lens = [int(L.svbrdf_desc_conv1_loss_partials(v, h, w))]
+            lens += [self._feature_partials(k) for k in range(1, len(self.hooks))]
+            buf = torch.empty(sum(lens), device=self.device, dtype=torch.float32)
+            hook = (torch.empty_like(y16), lens, buf)
             N.check(L.svbrdf_desc_conv1_loss(x.data_ptr(), p["w32"].data_ptr(), p["b"].data_ptr(), y16.data_ptr(), v, h,
                                              w, int(self.downsample), t32.data_ptr(), self._feature_coef(0, cf),
                                              hook[0].data_ptr(), buf.data_ptr(), st))
@@ -233,17 +233,39 @@ class VGGDescriptor:
         wt = self.hook_weights[k]
         return 2.0 * wt * wt * cf / sum(t.numel() for t in self.target[0])
 
+    def _pool_hooks(self):
+        """The hooks whose feature term runs in the backward pass of the pool above them: that
+        kernel reads the hook's feature anyway. Not with the Gram term, whose kernel carries it."""
+        if self.gram or self.fuse_pool:
+            return ()
+        return tuple(it[0] for it, above in zip(self.layers[1:], self.layers[2:])
+                     if above == "pool" and it != "pool" and it[0] in self.hooks)
+
+    def _feature_partials(self, k: int) -> int:
+        """The number of partial sums of hook k's feature term (no Gram term, k > 0)."""
+        if self.hooks[k] in self._pool_hooks():
+            return int(N.lib().svbrdf_desc_pool_bwd_loss_partials(*self.target[0][k].shape))
+        return int(N.lib().svbrdf_desc_partials())
+
     def _terms(self, hooks, cf: Optional[float], cg: Optional[float], hooks16=None):
         """Feature and Gram losses (0-d FP32 tensors). With cf/cg given, also the loss
         gradient at each hooked activation, cf d(feature)/df + cg d(gram)/df, as BF16 NHWC; the
         last layer's gradient is masked by its ReLU (it starts the backward chain). Every term's
         partial sums land in one buffer, and one launch (svbrdf_desc_loss_sums) adds them with
         the hook weights in a fixed order."""
+        grads, sums = self._term_grads(hooks, cf, cg, hooks16)
+        return *self._loss_sums(*sums), grads
+
+    def _term_grads(self, hooks, cf, cg, hooks16):
+        """(gradients, arguments of _loss_sums) of _terms. Where the forward pass has run
+        relu1_1's term, the terms of _pool_hooks are left to _backward: their gradient is (target,
+        coefficient, partial sums to fill), and _loss_sums has to wait for that pass."""
         L = N.lib()
         st = N.stream_handle(self.device)
         tf, tg = self.target
         # relu1_1's term where the forward pass has run it: (gradient, partial sums, all hooks' buffer)
         done = hooks["conv1_1"] if isinstance(hooks["conv1_1"], tuple) else None
+        late = self._pool_hooks() if done else ()
         if hooks16 is None:
             hooks16 = {n: (f if f.dtype == torch.bfloat16 else f.to(torch.bfloat16)) for n, f in hooks.items()}
         nf = sum(t.numel() for t in tf)
@@ -252,10 +274,10 @@ class VGGDescriptor:
         fused = cf is not None and self.gram
         # segments: each hook's feature partials, then each hook's Gram loss rows
         lens, weights, groups = [], [], []
-        for name, wt, t in zip(self.hooks, self.hook_weights, tf):
+        for k, (wt, t) in enumerate(zip(self.hook_weights, tf)):
             v, h, w, c = t.shape
             lens.append(int(L.svbrdf_desc_gemm_nt_feat_partials(v, h * w, c)) if fused else
-                        done[1] if done and name == "conv1_1" else nparts)
+                        done[1][k] if done else nparts)
             weights.append(wt * wt / nf)
             groups.append(0)
         if self.gram:
@@ -288,6 +310,9 @@ class VGGDescriptor:
                 rows = buf[offs[nh + k]:offs[nh + k] + lens[nh + k]].view(v, c)
                 _, _, dgram = gram_bf16(ff, self.err, tg[k], coef_g, want_dgram=cf is not None, rows_out=rows)
             coef = (2.0 * wt * wt * cf / nf) if cf is not None else 0.0
+            if name in late:
+                grads[name] = (self.target16[k], coef, part)
+                continue
             if cf is not None:
                 g = torch.empty(v, h, w, c, device=self.device, dtype=torch.bfloat16)
                 grads[name] = g
@@ -304,6 +329,12 @@ class VGGDescriptor:
             else:
                 N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), dtypes, t.data_ptr(), None, coef,
                                                 int(name == last), N.ptr(g), part.data_ptr(), f.numel(), st))
+        return grads, (buf, offs, lens, weights, groups)
+
+    def _loss_sums(self, buf, offs, lens, weights, groups):
+        """(feature loss, Gram loss): the weighted sums of the terms' partial sums."""
+        L = N.lib()
+        st = N.stream_handle(self.device)
         out = torch.empty(2, device=self.device, dtype=torch.float32)
         ns = len(lens)
         a_off = (ctypes.c_longlong * ns)(*offs)
@@ -314,7 +345,7 @@ class VGGDescriptor:
                                         ctypes.addressof(a_w), ctypes.addressof(a_g), out.data_ptr(), st))
         fl = out[0]
         gl = out[1] if self.gram else torch.zeros((), device=self.device)
-        return fl, gl, grads
+        return fl, gl
 
     # ---- backward chain ----------------------------------------------------------------
     def _backward(self, acts, grads, render_shape):
@@ -339,6 +370,14 @@ class VGGDescriptor:
                 # below is a convolution: route, add its hook gradient, mask by its ReLU
                 gx = torch.empty_like(x)
                 add = grads.get(below[0])
+                if isinstance(add, tuple):  # the hook's feature term runs here (_pool_hooks)
+                    t16, coef, part = add
+                    N.check(L.svbrdf_desc_pool_bwd_loss(g.data_ptr(), x.data_ptr(), t16.data_ptr(), coef,
+                                                        gx.data_ptr(), part.data_ptr(), n_, h, w, c,
+                                                        int(self.avg_pool), st))
+                    g = gx
+                    i -= 1
+                    continue
                 N.check(pool_bwd(g.data_ptr(), x.data_ptr(), N.ptr(add), gx.data_ptr(), n_, h, w, c, st))
                 g = gx
                 i -= 1
@@ -416,8 +455,9 @@ class VGGDescriptor:
 
     def _loss_and_grad_eager(self, renders):
         acts, hooks = self._forward(renders, None if self.gram else 1.0)
-        fl, gl, grads = self._terms(hooks, 1.0, 1.0, self._bf16_hooks(acts, hooks))
-        return fl, gl, self._backward(acts, grads, renders.shape)
+        grads, sums = self._term_grads(hooks, 1.0, 1.0, self._bf16_hooks(acts, hooks))
+        dr = self._backward(acts, grads, renders.shape)
+        return *self._loss_sums(*sums), dr
 
     def loss_and_grad(self, renders: torch.Tensor):
         """(feature_loss, gram_loss, d(feature + gram)/d renders) by one graph replay. The

@@ -547,3 +547,31 @@ def test_conv1_bwd_tc_widths_and_strips(svb, cuda, v, h, w, down):
     assert not torch.isnan(dr).any()
     assert rel_l2(dr, want) <= 1e-5
     assert float((dr.cpu().double() - want).abs().max()) <= 1e-4 * float(want.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 2, 2, 8), (2, 8, 12, 16), (3, 16, 66, 64), (1, 34, 128, 24)])
+@pytest.mark.parametrize("avg", [0, 1])
+def test_pool_bwd_loss_equals_its_two_kernels(svb, cuda, shape, avg):
+    """A pool's backward pass with the hook's feature term in it against the feature-loss kernel and
+    the pool's own, from one window to rows of several blocks and a remainder: the gradient equal, the
+    squared sum (FP32, another order over at most 64 x 6336 terms) within 1e-5."""
+    v, h, w, c = shape
+    N, L = svb._native, svb._native.lib()
+    gen = torch.Generator(device=cuda).manual_seed(h * w)
+    x, t, gy = (torch.randn(s, generator=gen, device=cuda).to(torch.bfloat16)
+                for s in (shape, shape, (v, h // 2, w // 2, c)))
+    x = torch.relu(x)
+    add, ga, gb = (torch.empty_like(x) for _ in range(3))
+    pa = torch.zeros(L.svbrdf_desc_partials(), device=cuda)
+    pb = torch.zeros(L.svbrdf_desc_pool_bwd_loss_partials(v, h, w, c), device=cuda)
+    st = N.stream_handle(cuda)
+    N.check(L.svbrdf_desc_feat_loss(x.data_ptr(), 3, t.data_ptr(), None, 0.37, 0, add.data_ptr(), pa.data_ptr(),
+                                    x.numel(), st))
+    plain = L.svbrdf_desc_avgpool_bwd if avg else L.svbrdf_desc_pool_bwd
+    N.check(plain(gy.data_ptr(), x.data_ptr(), add.data_ptr(), ga.data_ptr(), v, h, w, c, st))
+    N.check(L.svbrdf_desc_pool_bwd_loss(gy.data_ptr(), x.data_ptr(), t.data_ptr(), 0.37, gb.data_ptr(),
+                                        pb.data_ptr(), v, h, w, c, avg, st))
+    assert torch.equal(ga, gb)
+    a, b = pa.double().sum(), pb.double().sum()
+    assert abs(float(a - b)) <= 1e-5 * float(a)
