@@ -494,11 +494,12 @@ desc_feat_loss_kernel(const TF* __restrict__ f, const TT* __restrict__ t, const 
 // ---------------------------------------------------------------- loss sums
 // out[j] = sum over segments s of group j of w_s x (sum of the segment's floats), added in a
 // fixed order by one block. The segments are cut into units of 256 floats; warp w takes units w,
-// w + 32, ..., three at a time, eight loads a lane each, and adds its share of a segment in FP32
-// (a few dozen terms a lane, then a shuffle tree). The warps' shares are added and weighted in
-// double, one warp per segment: a double-precision instruction holds this part's FP64 pipe for 16
-// cycles a warp, and with every thread keeping its totals in double those instructions were the
-// kernel's 14 us (8 segments, 46,000 floats; 8.4 us so).
+// w + 32, ..., three at a time, eight loads a lane each, and a lane adds its terms of a segment in
+// FP32 (a few dozen). The lanes' totals are added as FP32 pairs (sum, rounding error), so that the
+// warp's share is as good as in double, and the shares are added and weighted in double, one warp
+// per segment: a double-precision instruction holds this part's FP64 pipe for 16 cycles a warp, and
+// with every thread keeping its totals in double those instructions were the kernel's 14 us
+// (8 segments, 46,000 floats; about 10 us so).
 constexpr int kMaxLossSegs = 16;
 constexpr int kLossSumThreads = 1024;
 struct LossSegs {
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(kLossSumThreads) desc_loss_sums_kernel(const f
                                                                           float* __restrict__ out) {
   constexpr int kWarps = kLossSumThreads / 32, kU = 3;  // units of a warp in flight
   static_assert(kWarps == 32 && kMaxLossSegs <= kWarps, "one lane per warp's share, one warp per segment");
-  __shared__ float share[kMaxLossSegs][kWarps];
+  __shared__ float2 share[kMaxLossSegs][kWarps];
   __shared__ double total[kMaxLossSegs];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   long long unit = warp;  // of this warp, counted from the start of segment k
@@ -535,13 +536,21 @@ __global__ void __launch_bounds__(kLossSumThreads) desc_loss_sums_kernel(const f
     }
     while (unit >= units + kWarps) unit -= kWarps;  // the first of its units past the segment's end
     unit -= units;
+    float lo = 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, o);
-    if (lane == 0) share[k][warp] = sk;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float b = __shfl_xor_sync(0xffffffffu, sk, o), bl = __shfl_xor_sync(0xffffffffu, lo, o);
+      const float s = sk + b, bb = s - sk;  // Knuth's two-sum: s + e = sk + b exactly
+      lo += bl + ((sk - (s - bb)) + (b - bb));
+      sk = s;
+    }
+    if (lane == 0) share[k][warp] = make_float2(sk, lo);
   }
   __syncthreads();
   if (warp < segs.n) {
-    double t = (double)share[warp][lane];
+    const float2 sh = share[warp][lane];
+    // an infinite sum has no rounding error to add (it reads NaN)
+    double t = (double)sh.x + (fabsf(sh.x) <= 3.402823466e+38f ? (double)sh.y : 0.0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) total[warp] = segs.w[warp] * t;
