@@ -387,3 +387,35 @@ def test_texel_pair_plan_shares(svb, lib, shapes, threads, ctas, variant):
     cta_run, mat_run = ints(hdr[19], n_ctas + 1), ints(hdr[20], len(shapes) + 1)
     assert [sum(s < cta[c] for s in starts) for c in range(n_ctas + 1)] == cta_run.tolist()
     assert [sum(seq[s][1] < m for s in starts) for m in range(len(shapes) + 1)] == mat_run.tolist()
+
+
+@pytest.mark.parametrize("shapes", [[(200, 200, 7)] * 24, [(300, 300, 3), (150, 150, 16), (38, 52, 9)] * 8, [(512, 512, 9)]])
+@pytest.mark.parametrize("threads,ctas,variant", [(480, 152, 3), (224, 20, 2), (384, 7, 3)])
+def test_texel_pair_plan_tile_cost(svb, lib, shapes, threads, ctas, variant):
+    """Shares of more than two tiles count 128 texels for each tile: every texel is dealt once, and no
+    CTA's cost, with its tiles', is above the mean by more than what a share can leave unused, a
+    step of 64 texels and one tile's cost (and half of that for where the last share ends)."""
+    SV = svb._native
+    mats, keep = _materials(SV, shapes)
+    cfg = SV.svbrdf_batch_config(threads, 2 * threads, ctas, variant)
+    nbytes = lib.svbrdf_batched_plan_bytes(mats, len(shapes), ctypes.byref(cfg))
+    buf = np.zeros(nbytes, np.uint8)
+    assert lib.svbrdf_batched_plan(mats, len(shapes), ctypes.byref(cfg), buf.ctypes.data, nbytes) == 0
+    hdr = np.frombuffer(buf[:84].tobytes(), np.int32)
+    n_tiles, n_ctas, off_cta, off_seq = hdr[2], hdr[3], hdr[8], hdr[16]
+    cta = np.frombuffer(buf[off_cta:off_cta + 4 * (n_ctas + 1)].tobytes(), np.int32)
+    seq = np.frombuffer(buf[off_seq:off_seq + 16 * n_tiles].tobytes(), np.int32).reshape(-1, 4)
+    assert cta[0] == 0 and cta[-1] == n_tiles and (np.diff(cta) >= 0).all()
+    counts = []
+    for m, (h, w, _) in enumerate(shapes):
+        first = [int(s[2]) for s in seq if s[1] == m]
+        assert first[0] == 0 and all(f % 64 == 0 for f in first)
+        n = np.diff(first + [h * w])
+        assert (n > 0).all() and (n <= 2 * threads).all()
+        counts += n.tolist()
+    assert len(counts) == n_tiles
+    texels = sum(h * w for h, w, _ in shapes)
+    extra = 128 if texels > 4 * threads * n_ctas else 0
+    cost = [(c + extra) * (shapes[s[1]][2] + 5.0) for c, s in zip(counts, seq)]
+    loads = [sum(cost[cta[c]:cta[c + 1]]) for c in range(n_ctas)]
+    assert max(loads) <= sum(loads) / n_ctas + 1.5 * (64 + extra) * (max(v for _, _, v in shapes) + 5.0)
