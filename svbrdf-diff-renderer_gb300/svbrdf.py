@@ -32,6 +32,21 @@ from . import _native as N
 LOSS_KINDS = {"mse": 0, "log1p": 1, "log1p_pre": 2}
 
 
+def _mark(t):
+    """What tells whether ``t`` has been written since: its version counter, or a copy of its values
+    where it keeps none (an inference tensor)."""
+    return t.clone() if t.is_inference() else t._version
+
+
+def _unwritten(t, was, mark):
+    """Whether ``t`` is the tensor ``was``, with the values that it had at ``mark``."""
+    return t is was and (torch.equal(t, mark) if torch.is_tensor(mark) else t._version == mark)
+
+
+def _same_memory(a, b):
+    return a.data_ptr() == b.data_ptr() and a.dtype == b.dtype and a.stride() == b.stride()
+
+
 class SvbrdfOptim:
     def __init__(self, device, renderer_obj, loss="mse", fused=True, graph=False, save_process=False,
                  descriptor=None, descriptor_weight=0.1, kernel="batched"):
@@ -203,14 +218,25 @@ class SvbrdfOptim:
         sc = Scene(res=H, size=float(r.size), camera_pos=r._cam, light_pos=r._lit,
                    light_pow=lp.detach().to(self.device, torch.float32), gt=None, targets=self.targets, init=tex)
         n = max(epochs, 1)
-        # A repeated call on the same maps, targets and settings reuses the previous call's plan,
-        # buffers and captured graph; every call still starts a fresh Adam (src/svbrdf.py:48-52).
-        key = (tex.data_ptr(), tuple(tex.shape), self.targets.data_ptr(), tuple(self.targets.shape), float(lr),
-               self.loss, bool(optim_light), n, r._cam.data_ptr(), r._lit.data_ptr(), float(r.size))
+        # A repeated call on the same maps and settings reuses the previous call's plan, buffers and
+        # captured graph; every call still starts a fresh Adam (src/svbrdf.py:48-52). The plan holds
+        # the maps by address (they stay alive with it), the views' positions by value, and the
+        # targets by address where the MSE loss takes the tensor as it is, else as a copy.
+        key = (tex.data_ptr(), tuple(tex.shape), tuple(self.targets.shape), float(lr), self.loss, bool(optim_light),
+               n, float(r.size))
         b = self._batched if getattr(self, "_batched_key", None) == key else None
-        if b is not None:  # the light may have changed since (update_light, or the last call's optim_light)
+        if b is not None and not all(_unwritten(t, *was) for t, was in zip((r._cam, r._lit), self._batched_views)):
+            b = None
+        if b is not None and not self._batched_copies and not _same_memory(self.targets, b.tgt[0]):
+            b = None
+        if b is not None:
+            # the light may have changed since (update_light, or the last call's optim_light), and the
+            # targets behind a copy may have been refilled or replaced
             b.lpow0[0].copy_(sc.light_pow)
             b.lpow[0].copy_(sc.light_pow)
+            if self._batched_copies:
+                tgt = self.targets.detach().to(self.device, torch.float32)
+                torch.log1p(tgt, out=b.tgt[0]) if self.loss == "log1p" else b.tgt[0].copy_(tgt)
             b.prepare(new_targets=False)
         else:
             # the texel-pair kernels (the resident-state one first) suit one material; the
@@ -219,6 +245,8 @@ class SvbrdfOptim:
             b = BatchedOptim([sc], lr=lr, loss=self.loss, device=self.device, hist_len=n, optim_light=optim_light,
                              adopt_maps=True, candidates=cands)
             self._batched, self._batched_key = b, key
+            self._batched_copies = not _same_memory(self.targets, b.tgt[0])
+            self._batched_views = [(t, _mark(t)) for t in (r._cam, r._lit)]
         tmp_dir = self._save_dir(svbrdf_obj)
         if tmp_dir is None:
             if epochs > 0:

@@ -113,3 +113,48 @@ def test_repeated_calls_start_fresh(svb, golden, cuda, light):
     assert max(abs(a - b) / b for a, b in zip(o.loss_image_list, second["loss"])) <= 1e-5
     if light:
         assert rel_l2(obj.cl[2].detach(), second["light_pow"]) <= 1e-6
+
+
+@pytest.mark.parametrize("change", ["refill", "load", "load_half", "camera", "light"])
+@pytest.mark.parametrize("loss", ["mse", "log1p"])
+def test_repeated_call_sees_new_targets_and_views(svb, cuda, loss, change):
+    """What a second optim call fits is what the optimiser holds then: targets refilled in place,
+    loaded anew (the old ones freed, so that their address can come back) or given in another type,
+    cameras and lights moved in place. Equal to a new optimiser's, bit for bit."""
+    from oracle import microfacet_ref as R
+    sc = svb.scenes.single_scene(res=32, seed=1031)
+    svb.scenes.add_targets(sc, lambda *a: R.render(*a, dtype=torch.float32))
+    other = (0.7 * sc.targets + 0.05).flip(0)
+    r = svb.Microfacet(32, 9, sc.size, [t.to(cuda) for t in sc.cl], cuda)
+
+    def fresh(targets):
+        o = svb.SvbrdfOptim(cuda, r, loss=loss)
+        o.load_targets(targets)
+        o.init_from_tex(sc.init.to(cuda))
+        return o
+
+    held = sc.targets.to(cuda)
+    o = fresh(held)
+    if change == "load_half":
+        o.targets = held.half()
+    o.optim(4, 0.01, None, False)
+    if change == "refill":
+        held.copy_(other)
+    elif change == "load":
+        del held
+        o.targets = None
+        o.load_targets(other.to(cuda))
+    elif change == "load_half":
+        o.targets = other.to(cuda).half()
+    elif change == "camera":
+        r._cam.mul_(1.1)
+    else:
+        r._lit.add_(0.5)
+    with torch.no_grad():
+        o.textures.copy_(sc.init)
+    o.optim(4, 0.01, None, False)
+    now = sc.targets if change in ("camera", "light") else other
+    n = fresh((now.half() if change == "load_half" else now).to(cuda))
+    n.optim(4, 0.01, None, False)
+    assert o.loss_image_list == n.loss_image_list
+    assert torch.equal(o.textures.detach(), n.textures.detach())
