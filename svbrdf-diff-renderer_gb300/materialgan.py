@@ -1015,8 +1015,9 @@ class MaterialGANOptim:
 
     def _graph_for(self, phase_latent: bool, lr: float):
         key = (phase_latent, float(lr))
-        if key in self._graphs:
-            return self._graphs[key]
+        light = getattr(self.renderer_obj, "light_pow", None)  # the graph reads it at its address
+        if key in self._graphs and self._graphs[key][3] is light:
+            return self._graphs[key][:3]
         params = [self.latent] if phase_latent else self.noises
         opt = torch.optim.Adam(params, lr=lr, betas=(0.9, 0.999), capturable=True)
         for p in params:
@@ -1036,8 +1037,8 @@ class MaterialGANOptim:
                 st["exp_avg"].zero_()
                 st["exp_avg_sq"].zero_()
             opt.step()
-        self._graphs[key] = (graph, loss, opt)
-        return self._graphs[key]
+        self._graphs[key] = (graph, loss, opt, light)
+        return graph, loss, opt
 
     def optim(self, epochs, lr, svbrdf_obj=None, optim_light=False, reset_adam_each_iter=True, graph=True):
         """``epochs = [total, l, n]``: alternate l latent epochs and n noise epochs. With

@@ -112,6 +112,27 @@ def test_latent_graph_matches_eager(svb, cuda):
 
 
 @pytest.mark.gpu
+def test_latent_graph_follows_a_new_light(svb, cuda):
+    """An epoch captured under one light power is not replayed under another: the loss of the epoch
+    after update_light is that of a render with the new light (same parameters, no step in
+    between; 1e-4 for the roundings of two passes, the light changes it severalfold)."""
+    gen = _small_gen(svb)
+    sc = svb.scenes.single_scene(res=32, seed=1016)
+    r = svb.Microfacet(32, 9, sc.size, [t.to(cuda) for t in sc.cl], cuda)
+    o = svb.materialgan.MaterialGANOptim(cuda, r, gen)
+    o.load_targets(torch.rand(9, 3, 32, 32, generator=torch.Generator().manual_seed(1)).to(cuda))
+    o.init_from(batch=1, seed=3)
+    old = r.light_pow
+    for light in (None, old * 3, old * 0.2):
+        if light is not None:
+            r.update_light(light)
+        with torch.no_grad():
+            want = float(o.compute_image_loss(r.eval(o.latent_to_textures())))
+        o.optim([1, 1, 0], 0.02)
+        assert abs(o.loss_image_list[-1] - want) <= 1e-4 * want
+
+
+@pytest.mark.gpu
 def test_refinement_handoff(svb, cuda):
     """Generator maps at 256 -> Lanczos 512 -> batched fused per-pixel refinement."""
     from oracle import microfacet_ref as R
