@@ -190,20 +190,18 @@ class VGGDescriptor:
         L = N.lib()
         st = N.stream_handle(self.device)
         x = renders.detach().float().contiguous()
-        v, _, rh, rw = x.shape
-        h, w = (rh // 2, rw // 2) if self.downsample else (rh, rw)
+        v, h, w = self._conv1_size(x.shape)
         p = self.params["conv1_1"]
         y16 = torch.empty(v, h, w, 64, device=self.device, dtype=torch.bfloat16)
         if cf is not None:
+            shapes = self._hook_shapes(v, h, w)
             t32 = self.target[0][0]
-            if tuple(t32.shape) != (v, h, w, 64):
-                raise ValueError(f"renders give {(v, h, w, 64)} features, the loaded targets {tuple(t32.shape)}")
             lens = [int(L.svbrdf_desc_conv1_loss_partials(v, h, w))]
-            lens += [self._feature_partials(k) for k in range(1, len(self.hooks))]
+            lens += [self._feature_partials(k, shapes[k]) for k in range(1, len(self.hooks))]
             buf = torch.empty(sum(lens), device=self.device, dtype=torch.float32)
             hook = (torch.empty_like(y16), lens, buf)
             N.check(L.svbrdf_desc_conv1_loss(x.data_ptr(), p["w32"].data_ptr(), p["b"].data_ptr(), y16.data_ptr(), v, h,
-                                             w, int(self.downsample), t32.data_ptr(), self._feature_coef(0, cf),
+                                             w, int(self.downsample), t32.data_ptr(), self._feature_coef(0, cf, shapes),
                                              hook[0].data_ptr(), buf.data_ptr(), st))
         else:
             hook = torch.empty(v, h, w, 64, device=self.device, dtype=torch.float32)
@@ -228,10 +226,32 @@ class VGGDescriptor:
         return acts, hooks
 
     # ---- loss terms --------------------------------------------------------------------
-    def _feature_coef(self, k: int, cf: float) -> float:
+    def _conv1_size(self, shape):
+        """(views, height, width) of the maps that conv1_1 sees for renders of ``shape``."""
+        v, _, h, w = shape
+        return (v, h // 2, w // 2) if self.downsample else (v, h, w)
+
+    def _hook_shapes(self, v: int, h: int, w: int):
+        """The hooked features' shapes of v renders that conv1_1 sees at h x w. The kernels read the
+        loaded targets at the same elements, so these have to have the same maps and at least as
+        many views (fewer renders are compared with the first targets)."""
+        shapes, c = [], 0
+        for item in self.layers:
+            if item == "pool":
+                h, w = h // 2, w // 2
+            else:
+                c = item[2]
+                if item[0] in self.hooks:
+                    shapes.append((v, h, w, c))
+        for name, s, t in zip(self.hooks, shapes, self.target[0]):
+            if s[1:] != tuple(t.shape[1:]) or s[0] > t.shape[0]:
+                raise ValueError(f"{name}: the renders give features {s}, the loaded targets {tuple(t.shape)}")
+        return shapes
+
+    def _feature_coef(self, k: int, cf: float, shapes) -> float:
         """cf d(feature loss)/d(f - t) of hook k, per unit of f - t: 2 w_k^2 / (all hooks' elements)."""
         wt = self.hook_weights[k]
-        return 2.0 * wt * wt * cf / sum(t.numel() for t in self.target[0])
+        return 2.0 * wt * wt * cf / sum(math.prod(s) for s in shapes)
 
     def _pool_hooks(self):
         """The hooks whose feature term runs in the backward pass of the pool above them: that
@@ -241,10 +261,10 @@ class VGGDescriptor:
         return tuple(it[0] for it, above in zip(self.layers[1:], self.layers[2:])
                      if above == "pool" and it != "pool" and it[0] in self.hooks)
 
-    def _feature_partials(self, k: int) -> int:
+    def _feature_partials(self, k: int, shape) -> int:
         """The number of partial sums of hook k's feature term (no Gram term, k > 0)."""
         if self.hooks[k] in self._pool_hooks():
-            return int(N.lib().svbrdf_desc_pool_bwd_loss_partials(*self.target[0][k].shape))
+            return int(N.lib().svbrdf_desc_pool_bwd_loss_partials(*shape))
         return int(N.lib().svbrdf_desc_partials())
 
     def _terms(self, hooks, cf: Optional[float], cg: Optional[float], hooks16=None):
@@ -260,29 +280,28 @@ class VGGDescriptor:
         """(gradients, arguments of _loss_sums) of _terms. Where the forward pass has run
         relu1_1's term, the terms of _pool_hooks are left to _backward: their gradient is (target,
         coefficient, partial sums to fill), and _loss_sums has to wait for that pass."""
+        # relu1_1's term where the forward pass has run it: (gradient, partial sums, all hooks' buffer)
+        done = hooks["conv1_1"] if isinstance(hooks["conv1_1"], tuple) else None
+        shapes = self._hook_shapes(*(done[0] if done else hooks["conv1_1"]).shape[:3])
         L = N.lib()
         st = N.stream_handle(self.device)
         tf, tg = self.target
-        # relu1_1's term where the forward pass has run it: (gradient, partial sums, all hooks' buffer)
-        done = hooks["conv1_1"] if isinstance(hooks["conv1_1"], tuple) else None
         late = self._pool_hooks() if done else ()
         if hooks16 is None:
             hooks16 = {n: (f if f.dtype == torch.bfloat16 else f.to(torch.bfloat16)) for n, f in hooks.items()}
-        nf = sum(t.numel() for t in tf)
+        nf = sum(math.prod(s) for s in shapes)
         ng = sum(g.numel() for g in tg)
         nparts = L.svbrdf_desc_partials()
         fused = cf is not None and self.gram
         # segments: each hook's feature partials, then each hook's Gram loss rows
         lens, weights, groups = [], [], []
-        for k, (wt, t) in enumerate(zip(self.hook_weights, tf)):
-            v, h, w, c = t.shape
+        for k, (wt, (v, h, w, c)) in enumerate(zip(self.hook_weights, shapes)):
             lens.append(int(L.svbrdf_desc_gemm_nt_feat_partials(v, h * w, c)) if fused else
                         done[1][k] if done else nparts)
             weights.append(wt * wt / nf)
             groups.append(0)
         if self.gram:
-            for name, wt, t in zip(self.hooks, self.hook_weights, tf):
-                v, h, w, c = t.shape
+            for wt, (v, h, w, c) in zip(self.hook_weights, shapes):
                 lens.append(v * c)
                 weights.append(wt * wt / ng)
                 groups.append(1)
@@ -432,6 +451,7 @@ class VGGDescriptor:
         """(feature_loss, gram_loss) as 0-d tensors, differentiable w.r.t. ``renders``."""
         if self.target is None:
             raise RuntimeError("call load(targets) first")
+        self._hook_shapes(*self._conv1_size(renders.shape))
         return _DescriptorLoss.apply(renders, self)
 
     def device_error(self) -> int:
@@ -465,6 +485,7 @@ class VGGDescriptor:
         if self.target is None:
             raise RuntimeError("call load(targets) first")
         if getattr(self, "_graph", None) is None or self._graph[0] != tuple(renders.shape):
+            self._hook_shapes(*self._conv1_size(renders.shape))
             self._capture(renders.shape)
         _, graph, static_r, fl, gl, dr = self._graph
         with torch.no_grad():

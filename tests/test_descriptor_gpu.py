@@ -575,3 +575,30 @@ def test_pool_bwd_loss_equals_its_two_kernels(svb, cuda, shape, avg):
     assert torch.equal(ga, gb)
     a, b = pa.double().sum(), pb.double().sum()
     assert abs(float(a - b)) <= 1e-5 * float(a)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["config", "reference"])
+def test_renders_of_other_shapes_than_the_targets(svb, cuda, mode):
+    """Renders of other maps or more views than the targets' are refused by both entry points; fewer
+    views equal a descriptor that holds the first targets alone, in losses (one fixed-order sum
+    in FP32: 1e-6) and gradient. The Gram loss stays a mean over all loaded targets."""
+    make = lambda: svb.descriptor.VGGDescriptor(cuda, seed=2, mode=mode)
+    gen = torch.Generator().manual_seed(7)
+    res = 256 if mode == "config" else 128
+    tgt, cur = (torch.rand(3, 3, res, res, generator=gen).to(cuda) for _ in range(2))
+    d, first = make(), make()
+    d.load(tgt)
+    first.load(tgt[:2])
+    for v, r in ((4, res), (3, 2 * res), (3, res // 2)):
+        wrong = torch.rand(v, 3, r, r, generator=gen).to(cuda)
+        with pytest.raises(ValueError):
+            d.loss(wrong)
+        with pytest.raises(ValueError):
+            d.loss_and_grad(wrong)
+    for a, b in zip((d.loss(cur[:2]), d.loss_and_grad(cur[:2])), (first.loss(cur[:2]), first.loss_and_grad(cur[:2]))):
+        assert abs(float(a[0]) - float(b[0])) <= 1e-6 * float(b[0])
+        assert abs(float(a[1]) - float(b[1]) * 2 / 3) <= 1e-6 * float(b[1])
+    if mode == "reference":
+        assert torch.equal(d.loss_and_grad(cur[:2])[2], first.loss_and_grad(cur[:2])[2])
+    assert d.device_error() == 0

@@ -1,6 +1,7 @@
 """The FP64 descriptor oracle on the CPU: its two modes follow the stacks they restate."""
 import math
 
+import pytest
 import torch
 
 from oracle import descriptor_ref as DR
@@ -96,3 +97,27 @@ def test_reference_mode_matches_reference_vggloss(golden):
     g = grad.reshape(-1)
     assert torch.allclose(g[d["grad_idx"].long()], d["grad_val"], rtol=1e-9, atol=1e-15)
     assert abs(float(grad.norm()) - float(d["grad_norm"])) <= 1e-10 * float(d["grad_norm"])
+
+
+@pytest.mark.parametrize("mode", ["config", "reference"])
+@pytest.mark.parametrize("views,res,ok", [(2, 256, True), (1, 256, True), (3, 256, False), (2, 128, False),
+                                          (2, 512, False)])
+def test_renders_have_to_fit_the_loaded_targets(svb, mode, views, res, ok):
+    """The kernels read the targets' features at the renders' elements: other maps or more views than
+    were loaded are refused before a launch, fewer views are compared with the first targets."""
+    d = svb.descriptor.VGGDescriptor("cpu", mode=mode)
+    at = lambda v, r: (v, r // 2, r // 2) if d.downsample else (v, r, r)
+    shapes = {}
+    for v, r in {(2, 256), (views, res)}:
+        _, h, w = at(v, r)
+        div = {"conv1_1": 1, "conv1_2": 1, "conv3_2": 4, "conv4_1": 8, "conv4_2": 8}
+        ch = {"conv1_1": 64, "conv1_2": 64, "conv3_2": 256, "conv4_1": 512, "conv4_2": 512}
+        shapes[v, r] = [(v, h // div[n], w // div[n], ch[n]) for n in d.hooks]
+    meta = lambda ss: [torch.empty(s, device="meta") for s in ss]
+    d.target = (meta(shapes[2, 256]), [])
+    hooks = dict(zip(d.hooks, meta(shapes[views, res])))
+    if ok:
+        assert d._hook_shapes(*at(views, res)) == shapes[views, res]
+    else:
+        with pytest.raises(ValueError):
+            d._term_grads(hooks, None, None, None)
