@@ -574,6 +574,27 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, int* e
   return wait_phase_n(bar, parity, err, code, kSpinLimit);
 }
 
+// Bounded wait for a copy to land; unlike wait_phase it goes on when the error word is set.
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, int* err) {
+  uint32_t it = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if (++it >= kSpinLimit) { atomicCAS(err, 0, (int)kDevTimeoutDrain); break; }
+  }
+}
+
+// The producer's last act in a ring whose next free slot is (slot, phase): the copies of the last
+// min(R, issued) chunks land before the CTA's shared memory goes away. Consumers wait for every
+// chunk that they use, but one that gave up leaves chunks behind, also when the producer had
+// issued its last one by then and never saw a wait run out.
+__device__ __forceinline__ void drain_ring(uint64_t* full_bar, int R, int slot, uint32_t phase, long long issued,
+                                           int* err) {
+  const long long n = issued < R ? issued : R;
+  for (long long i = 0; i < n; ++i) {
+    if (--slot < 0) { slot = R - 1; phase ^= 1u; }
+    drain_wait(smem_u32(&full_bar[slot]), phase, err);
+  }
+}
+
 // Consumer-side ring cursor.
 struct RingCursor {
   int slot;
@@ -679,19 +700,7 @@ batched_tma_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restri
           if (++slot == R) { slot = 0; phase ^= 1u; }
         }
       }
-      if (!ok) {
-        // drain: wait for the copies of the last min(R, issued) chunks to land
-        const long long n = issued < R ? issued : R;
-        int s = slot;
-        uint32_t ph = phase;
-        for (long long i = 0; i < n; ++i) {
-          if (--s < 0) { s = R - 1; ph ^= 1u; }
-          uint32_t it = 0;
-          while (!mbar_try_wait(smem_u32(&full_bar[s]), ph)) {
-            if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-          }
-        }
-      }
+      drain_ring(full_bar, R, slot, phase, issued, err);
     }
   } else {
     // ------------------------------------------------------------ consumers
@@ -981,7 +990,6 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       // release that publishes the record); lanes 0 .. nplanes-1 then issue one plane copy
       // each. The next tile's entry is loaded one tile ahead and a material's fields and
       // views only when the material changes.
-      const bool was_ok = ok;
       int4 sq_next = sq_first;
       int run_tile = 0;
       for (int k = k0; k < k1 && ok; ++k) {
@@ -1051,19 +1059,6 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
                      bytes, fb);
           ++issued;
           if (++slot == R) { slot = 0; phase ^= 1u; }
-        }
-      }
-      if (!ok && was_ok && lane == 0) {
-        // drain: wait for the copies of the last min(R, issued) chunks to land
-        const long long n = issued < R ? issued : R;
-        int s = slot;
-        uint32_t ph = phase;
-        for (long long i = 0; i < n; ++i) {
-          if (--s < 0) { s = R - 1; ph ^= 1u; }
-          uint32_t it = 0;
-          while (!mbar_try_wait(smem_u32(&full_bar[s]), ph)) {
-            if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-          }
         }
       }
       __syncwarp();
@@ -1272,6 +1267,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     if (more && !batched_next_iteration(last, ws, number0 + 1 + it, &s_last)) break;
     if (more) asm volatile("fence.proxy.async;" ::: "memory");
   }
+  if (warp == NCW && lane == 0) drain_ring(full_bar, R, slot, phase, issued, err);
 }
 
 // ============================================================== variant 3: resident state
@@ -1463,24 +1459,9 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         }
       }
     }
-    if (!ok && lane == 0) {
-      // drain: the last min(R, issued) ring chunks and the last state copy must land
-      const long long n = issued < R ? issued : R;
-      int s = slot;
-      uint32_t ph = phase;
-      for (long long i = 0; i < n; ++i) {
-        if (--s < 0) { s = R - 1; ph ^= 1u; }
-        uint32_t it = 0;
-        while (!mbar_try_wait(smem_u32(&full_bar[s]), ph)) {
-          if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-        }
-      }
-      if (states > 0) {
-        uint32_t it = 0;
-        while (!mbar_try_wait(sfull, (uint32_t)((states - 1) & 1))) {
-          if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-        }
-      }
+    if (lane == 0) {
+      drain_ring(full_bar, R, slot, phase, issued, err);
+      if (states > 0) drain_wait(sfull, (uint32_t)((states - 1) & 1), err);
     }
     __syncwarp();
   } else {
@@ -2000,18 +1981,9 @@ batched_fuse2_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __rest
   if (threadIdx.x == 0 && *(volatile int*)err != 0) {
     // drain: every copy this CTA issued must land before the CTA's shared memory goes away
     for (int s = 0; s < R; ++s) {
-      if (issue_cnt[s] == 0) continue;
-      uint32_t it = 0;
-      while (!mbar_try_wait(smem_u32(&full_bar[s]), (uint32_t)((issue_cnt[s] - 1) & 1))) {
-        if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-      }
+      if (issue_cnt[s] > 0) drain_wait(smem_u32(&full_bar[s]), (uint32_t)((issue_cnt[s] - 1) & 1), err);
     }
-    if (st_issued > 0) {
-      uint32_t it = 0;
-      while (!mbar_try_wait(smem_u32(&state_full), (uint32_t)((st_issued - 1) & 1))) {
-        if (++it >= kSpinLimit) { atomicCAS(err, 0, kDevTimeoutDrain); break; }
-      }
-    }
+    if (st_issued > 0) drain_wait(smem_u32(&state_full), (uint32_t)((st_issued - 1) & 1), err);
   }
   batched_finish<NT>(plan, hdr, mats, warp_loss, NCW, loss_hist, hist_len, s_step, step_counter,
                      ws + kWsCounter, &s_last, NCW, iters);

@@ -47,6 +47,26 @@ def test_host_turns_the_error_word_into_an_exception(svb, cuda):
         b.check()
 
 
+@pytest.mark.parametrize("variant", [1, 2, 3, 4])
+def test_launch_under_a_set_error_word_returns(svb, cuda, variant):
+    """Every wait of a launch whose workspace holds an error code may give up at once, with copies in
+    flight: the launch drains them, returns and keeps the code, and the next plan is healthy."""
+    off = svb._native.WORKSPACE_ERROR_OFFSET
+    cfg = svb.BatchConfig({1: 480, 2: 480, 3: 480, 4: 512}[variant], {1: 480, 4: 1024}.get(variant, 960), 0, variant)
+    b = svb.BatchedOptim(_mats(svb), device=cuda, config=cfg, hist_len=4)
+    b.ws[off:off + 4].view(torch.int32).fill_(2)
+    b.run(4)
+    assert b.device_error() == 2
+    runs = []
+    for _ in range(2):
+        c = svb.BatchedOptim(_mats(svb), device=cuda, config=cfg, hist_len=4)
+        c.run(4)
+        c.check()
+        runs.append(c)
+    assert torch.equal(runs[0].loss_hist, runs[1].loss_hist) and torch.isfinite(runs[0].loss_hist).all()
+    assert all(torch.equal(x, y) for x, y in zip(runs[0].tex, runs[1].tex))
+
+
 @pytest.mark.parametrize("variant", [2, 3])
 def test_batched_checkpoint_resume_is_exact(svb, cuda, tmp_path, variant):
     mats = _mats(svb)
