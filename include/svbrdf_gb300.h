@@ -182,8 +182,10 @@ typedef struct svbrdf_batch_config {
 /* Workspace of svbrdf_batched_step: the int32 at byte offset 4 is a device error word,
  * 0 while healthy. A pipelined launch that waited too long for its copies or consumers
  * stores a non-zero code there (1: copy never landed, 2: consumers stalled, 3: drain
- * timeout, 4: an iteration of a cooperative launch never ended in some CTA), skips the rest of its work and returns; the caller reads the word after
- * synchronising and treats non-zero as a failed step. */
+ * timeout, 4: an iteration of a cooperative launch never ended in some CTA), skips the rest
+ * of its work and returns; the caller reads the word after synchronising and treats non-zero
+ * as a failed step: maps, moments, light powers, loss rows and the step counter are then not
+ * valid. The workspace itself is, once the word has been zeroed. */
 #define SVBRDF_WORKSPACE_ERROR_OFFSET 4
 
 /* Self-test of the batched kernels' failure path: a one-warp kernel waits on an mbarrier

@@ -340,10 +340,16 @@ __device__ __forceinline__ void run_flush(RunSums* row, int run_tile, int n_tile
   __syncwarp();
 }
 
+// Counts the CTA in; 1 in the one that comes last of the grid. The counter wraps to zero by itself
+// with that arrival, so it is zero again whenever every CTA has come equally often.
+__device__ __forceinline__ int arrive_last(unsigned* counter) {
+  return atomicInc(counter, gridDim.x - 1) == gridDim.x - 1 ? 1 : 0;
+}
+
 // End of a launch (or of an iteration of a cooperative one), in every CTA: the warps' sums of
 // each of the CTA's runs are added into one total per run and quantity; the last CTA to finish
-// adds each material's run totals in run order, fills the loss history, steps the learnable
-// lights and resets the completion counter. Every level has a fixed order, so losses and lights
+// adds each material's run totals in run order, fills the loss history and steps the learnable
+// lights. Every level has a fixed order, so losses and lights
 // are deterministic. A warp forms one total with one load per lane and a shuffle tree, and the
 // last CTA reads one value per (run, quantity), at most one per CTA of each material: the tile
 // totals that this replaces took a serial sum over the warps, and one value per tile, and with
@@ -379,7 +385,7 @@ __device__ __forceinline__ bool run_finish(const char* plan, const PlanHeader* h
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    const int last = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1 : 0;
+    const int last = arrive_last(counter);
     if (last) __threadfence();
     *s_flag = last;
   }
@@ -409,10 +415,7 @@ __device__ __forceinline__ bool run_finish(const char* plan, const PlanHeader* h
     md.lstate[c] = m1;
     md.lstate[3 + c] = m2;
   }
-  if (threadIdx.x == 0) {
-    *step_counter = step;
-    *counter = 0u;
-  }
+  if (threadIdx.x == 0) *step_counter = step;
   return true;
 }
 
@@ -1264,7 +1267,14 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     if (more) asm volatile("fence.proxy.async;" ::: "memory");
     const bool last = run_finish<NCW>(plan, hdr, mats, s_sums, warp_loss, lpart, loss_hist, hist_len, step0 + 1 + it,
                                       step_counter, ws + kWsCounter, &s_last, 1, &s_adam[it]);
-    if (more && !batched_next_iteration(last, ws, number0 + 1 + it, &s_last)) break;
+    if (more && !batched_next_iteration(last, ws, number0 + 1 + it, &s_last)) {
+      // Given up, with the error word set. The CTAs leave at different iterations, so each still
+      // arrives for those that it does not run: a caller who zeroes the error word can use the
+      // workspace again. What the others make of these arrivals is as invalid as the launch.
+      if (threadIdx.x == 0)
+        for (int i = it + 1; i < iters; ++i) arrive_last(ws + kWsCounter);
+      break;
+    }
     if (more) asm volatile("fence.proxy.async;" ::: "memory");
   }
   if (warp == NCW && lane == 0) drain_ring(full_bar, R, slot, phase, issued, err);

@@ -67,6 +67,34 @@ def test_launch_under_a_set_error_word_returns(svb, cuda, variant):
     assert all(torch.equal(x, y) for x, y in zip(runs[0].tex, runs[1].tex))
 
 
+@pytest.mark.parametrize("ctas", [0, 5])
+@pytest.mark.parametrize("variant,light", [(2, True), (3, True), (2, False), (3, False)])
+def test_workspace_is_usable_again_once_the_word_is_zeroed(svb, cuda, variant, light, ctas):
+    """A launch that gave up (here because its workspace held an error code: with a learnable light
+    the CTAs of variant 2 leave at their first wait for one another, with iterations to go) leaves
+    no count behind: with the word zeroed and the fit reset, the same plan runs as a fresh one."""
+    off = svb._native.WORKSPACE_ERROR_OFFSET
+    make = lambda: svb.BatchedOptim(_mats(svb), device=cuda, config=svb.BatchConfig(480, 960, ctas, variant),
+                                    hist_len=9, optim_light=light)
+    b = make()
+    word = b.ws[off:off + 4].view(torch.int32)
+    for iters in (5, 1, 9):
+        word.fill_(2)
+        b.run(iters)
+        assert b.device_error() == 2
+        word.zero_()
+        assert int(b.ws[:4].view(torch.int32).item()) == 0  # the completion counter
+    b.reset(inits=[m.init for m in _mats(svb)])
+    b.run(9)
+    b.check()
+    c = make()
+    c.run(9)
+    c.check()
+    assert torch.equal(b.loss_hist, c.loss_hist)
+    for i in range(b.n):
+        assert torch.equal(b.tex[i], c.tex[i]) and torch.equal(b.light_pow(i), c.light_pow(i))
+
+
 @pytest.mark.parametrize("variant", [2, 3])
 def test_batched_checkpoint_resume_is_exact(svb, cuda, tmp_path, variant):
     mats = _mats(svb)
