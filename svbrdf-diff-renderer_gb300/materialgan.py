@@ -36,6 +36,18 @@ from . import _native as N
 LRELU_GAIN = math.sqrt(2.0)
 
 
+def _bare(m, cls) -> bool:
+    """Whether a call of module ``m`` is ``cls.forward`` and nothing else: no hook on it or on all
+    modules, no forward of its own. Only such a call may be replaced by something that computes
+    its result in another way."""
+    hooks = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+    every = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks",
+             "_global_backward_pre_hooks")
+    return (getattr(type(m), "forward", None) is cls.forward and "forward" not in vars(m)
+            and not any(getattr(m, h, None) for h in hooks)
+            and not any(getattr(torch.nn.modules.module, h, None) for h in every))
+
+
 def _nf(res: int, fmap_base: int = 16384, fmap_max: int = 512) -> int:
     """Channels of the block producing res^2: fmap_base / 2^(log2(res) - 1), capped."""
     return min(int(fmap_base * 2 / res), fmap_max)
@@ -613,7 +625,7 @@ class _ModConv(torch.nn.Module):
         """(the convolution's style-scaled, up-sampled input, demodulation, scaled weight, padding)."""
         wsc, w2t = self._scaled_weight()
         if sd is None:
-            sd = self._style(w, w2t)
+            sd = self._style(w, w2t, _use_kernels(x))
         s, d = sd  # [B, cin], [B, cout] or None
         # an up-sampling layer convolves the up-sampled map with its one-sample halo, unpadded
         # (_upsample2_halo): the reference's transposed convolution + filter on the border too
@@ -630,10 +642,12 @@ class _ModConv(torch.nn.Module):
                 x = _upsample2_halo(x)  # per-channel linear: commutes with the channel scaling
         return x, d, wsc, pad
 
-    def _style(self, w, w2t):
-        """(style, demodulation or None) of w [B, w_dim]."""
+    def _style(self, w, w2t, kernels=True):
+        """(style, demodulation or None) of w [B, w_dim]; without ``kernels`` (the layer's map takes
+        torch's operations) by torch's operations too."""
         aff = self.affine
-        if (_use_kernels(w) and w.dim() == 2 and aff.weight.dtype == torch.float32 and not aff.act and
+        if (kernels and _use_kernels(w) and w.dim() == 2 and _bare(aff, _Dense) and
+                aff.weight.dtype == torch.float32 and not aff.act and
                 not (self.weight.requires_grad or aff.weight.requires_grad or aff.bias.requires_grad)):
             return _StyleDemod.apply(w, *aff.scaled(), w2t if self.demod else None)
         s = aff(w)
@@ -887,14 +901,15 @@ class StyleGAN2Generator(torch.nn.Module):
             if fuse:
                 x = up(x, wp[:, 1 + 2 * i], n_up, sd.get(up.conv), s_next=sd[conv.conv][0])
                 # the last map feeds only its toRGB layer: its epilogue applies that style too, and
-                # the unscaled map is neither stored nor read again
-                last = i == len(self.ups) - 1 and rgb.conv in sd and rgb.kernel_ok(x, img)
-                x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv), prescaled=True,
-                         s_next=sd[rgb.conv][0] if last else None)
+                # the unscaled map is neither stored nor read again (unless someone looks at it)
+                last = (i == len(self.ups) - 1 and _bare(conv, _StyleLayer) and _bare(rgb, _ToRGB) and
+                        rgb.conv in sd and rgb.kernel_ok(x, img))
+                scale = {"s_next": sd[rgb.conv][0]} if last else {}
+                x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv), prescaled=True, **scale)
             else:
                 x = up(x, wp[:, 1 + 2 * i], n_up, sd.get(up.conv))
                 x = conv(x, wp[:, 2 + 2 * i], n_conv, sd.get(conv.conv))
-            img = rgb(x, wp[:, 3 + 2 * i], img, sd.get(rgb.conv), prescaled=last)
+            img = rgb(x, wp[:, 3 + 2 * i], img, sd.get(rgb.conv), **({"prescaled": True} if last else {}))
         return img
 
 

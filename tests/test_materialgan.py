@@ -628,3 +628,79 @@ def test_conv_act_equals_its_two_kernels(svb, cuda, shape, pad, with_noise, scal
     assert MG.generator_device_error(cuda) == 0
     for a, c in zip(*res):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("kind", ["hook", "pre", "global", "method", "module", "none"])
+def test_affine_of_a_layer_called_alone_is_called(svb, monkeypatch, kind):
+    """A frozen layer computes its style through conv.affine as a module where anything is attached to
+    it (a hook on it or on every module, a forward of its own, another module in its place), and
+    by the fused node otherwise, with the same values."""
+    M = svb.materialgan
+    monkeypatch.setattr(M, "_use_kernels", lambda t: True)
+    layer = _small_gen(svb).requires_grad_(False).convs[0].conv
+    w = torch.randn(2, 64, generator=torch.Generator().manual_seed(3))
+    w2t = layer._scaled_weight()[1]
+    want = layer.affine(w)
+    seen, handle = [], None
+    if kind == "hook":
+        handle = layer.affine.register_forward_hook(lambda m, a, out: seen.append(out))
+    elif kind == "pre":
+        handle = layer.affine.register_forward_pre_hook(lambda m, a: seen.append(a))
+    elif kind == "global":
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, a, out: seen.append(out))
+    elif kind == "method":
+        plain = layer.affine.forward
+        layer.affine.forward = lambda v: (seen.append(v), plain(v))[1]
+    elif kind == "module":
+        class Wrapped(torch.nn.Module):
+            def __init__(self, inner):
+                super().__init__()
+                self.inner, self.weight, self.bias = inner, inner.weight, inner.bias
+
+            def forward(self, v):
+                seen.append(v)
+                return self.inner(v)
+        layer.affine = Wrapped(layer.affine)
+    try:
+        s, d = layer._style(w, w2t)
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert bool(seen) == (kind != "none")
+    assert torch.equal(s, want) and torch.equal(d, torch.rsqrt(want.pow(2) @ w2t + 1e-8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["conv", "rgb", "affine"])
+def test_hooks_see_the_values_of_the_plain_layers(svb, cuda, where):
+    """A hook on the last style layer sees that layer's output, one on its toRGB layer that layer's
+    input (neither times the toRGB style), one on a frozen layer's affine fires when the layer is
+    called on its own; the image does not depend on their being there (TF32 convolutions of the
+    same operands either way: 1e-4)."""
+    gen = svb.materialgan.StyleGAN2Generator(resolution=32, w_dim=64, fmap_base=512, fmap_max=64, seed=0,
+                                             mapping_layers=2).to(cuda).requires_grad_(False)
+    wp = torch.randn(2, gen.num_ws, 64, generator=torch.Generator().manual_seed(5)).to(cuda)
+    plain = gen.synthesis(wp)
+    seen = []
+    if where == "affine":
+        layer = gen.convs[0]
+        x = torch.randn(2, layer.conv.weight.shape[1], 8, 8, device=cuda).to(memory_format=torch.channels_last)
+        want = layer.conv.affine(wp[:, 2])
+        with_out = layer(x, wp[:, 2], None)
+        layer.conv.affine.register_forward_hook(lambda m, a, out: seen.append(out))
+        assert rel_l2(layer(x, wp[:, 2], None), with_out) <= 1e-6
+        assert len(seen) == 1 and rel_l2(seen[0], want) <= 1e-6
+        return
+    ins, outs = [], []
+    if where == "conv":
+        gen.convs[-1].register_forward_hook(lambda m, a, out: outs.append(out.clone()))
+    gen.rgbs[-1].register_forward_pre_hook(lambda m, a: ins.append(a[0].clone()))
+    img = gen.synthesis(wp)
+    # toRGB of the map that the hooks saw, with the module's own style, is the image
+    skip = []
+    gen.rgbs[-2].register_forward_hook(lambda m, a, out: skip.append(out.clone()))
+    gen.synthesis(wp)
+    again = gen.rgbs[-1](ins[0], wp[:, gen.num_ws - 1], skip[0])
+    assert rel_l2(img, plain) <= 1e-4 and rel_l2(again, plain) <= 1e-4
+    if where == "conv":
+        assert torch.equal(outs[0], ins[0])
