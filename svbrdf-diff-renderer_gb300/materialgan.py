@@ -483,6 +483,7 @@ class _StyleDemod(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, w, a, bias, w2t):
+        ctx.set_materialize_grads(False)  # an unused output arrives as None, not as zeros
         s = Fn.linear(w, a, bias)
         d = torch.rsqrt(s.pow(2) @ w2t + 1e-8) if w2t is not None else None
         ctx.save_for_backward(s, d, a, w2t)

@@ -704,3 +704,31 @@ def test_hooks_see_the_values_of_the_plain_layers(svb, cuda, where):
     assert rel_l2(img, plain) <= 1e-4 and rel_l2(again, plain) <= 1e-4
     if where == "conv":
         assert torch.equal(outs[0], ins[0])
+
+
+@pytest.mark.parametrize("use", ["s", "d", "both"])
+def test_style_node_with_an_unused_output(svb, use):
+    """The style node's adjoint when only one of its outputs is used: autograd's gradient (FP64, 1e-12),
+    and no product with the squared weights where the demodulation has no gradient."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Products(TorchDispatchMode):
+        n = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.n += func in (torch.ops.aten.mm.default, torch.ops.aten.addmm.default)
+            return func(*args, **(kwargs or {}))
+
+    g = torch.Generator().manual_seed(2)
+    w, a, bias, w2t = (torch.randn(*s, generator=g, dtype=torch.float64) for s in ((3, 8), (6, 8), (6,), (6, 5)))
+    w2t, ws, wd = w2t.abs(), torch.randn(3, 6, generator=g, dtype=torch.float64), torch.randn(3, 5, generator=g, dtype=torch.float64)
+    loss = lambda s, d: (0 if use == "d" else (s * ws).sum()) + (0 if use == "s" else (d * wd).sum())
+    x = w.clone().requires_grad_(True)
+    s = torch.nn.functional.linear(x, a, bias)
+    loss(s, torch.rsqrt(s.pow(2) @ w2t + 1e-8)).backward()
+    y = w.clone().requires_grad_(True)
+    out = loss(*svb.materialgan._StyleDemod.apply(y, a, bias, w2t))
+    with Products() as seen:
+        out.backward()
+    assert rel_l2(y.grad, x.grad) <= 1e-12
+    assert seen.n == (1 if use == "s" else 2)
