@@ -727,6 +727,8 @@ class _ToRGB(torch.nn.Module):
         if self.kernel_ok(x, skip):
             yp, _ = self.conv.parts(x, w, keep_pad=True, sd=sd, prescaled=prescaled)
             return _RgbNHWC.apply(_cl(yp), self.bias, skip, self.bias.shape[0])
+        if prescaled:
+            raise ValueError("toRGB: a prescaled input needs the fused path (kernel_ok)")
         y = self.conv(x, w) + self.bias.view(1, -1, 1, 1)
         return y if skip is None else y + _upsample2(skip)
 

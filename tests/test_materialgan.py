@@ -732,3 +732,13 @@ def test_style_node_with_an_unused_output(svb, use):
         out.backward()
     assert rel_l2(y.grad, x.grad) <= 1e-12
     assert seen.n == (1 if use == "s" else 2)
+
+
+def test_torgb_refuses_a_prescaled_input_without_its_fused_path(svb):
+    """Outside the fused path toRGB applies its style to the input itself: a map that carries it
+    already would be scaled twice."""
+    rgb = _small_gen(svb).requires_grad_(False).rgbs[-1]
+    x, w = torch.randn(1, rgb.conv.weight.shape[1], 8, 8), torch.randn(1, 64)
+    assert rgb(x, w, None).shape == (1, 9, 8, 8)
+    with pytest.raises(ValueError):
+        rgb(x, w, None, prescaled=True)
