@@ -326,8 +326,9 @@ int svbrdf_desc_pool_bwd_loss(const void* gy, const void* x, const void* target,
 
 /* Feature term of one hook: partial[b] (b < svbrdf_desc_partials(), if partial) = block b's
  * share of sum (f - t)^2, a fixed-order split; if g: g = coef (f - t) + gram_grad (nullable),
- * times (f > 0) if `mask`, stored BF16. `dtypes` bit 0: f is BF16, else FP32; bit 1: t is BF16,
- * else FP32; gram_grad FP32; all n elements. */
+ * times (f > 0) if `mask`, stored BF16. `dtypes` 0: f and t are FP32, 1: f is BF16, 2: t is BF16,
+ * 3: both; any other value reads as 1 (the argument was a flag for f, whose 0 and 1 are unchanged);
+ * gram_grad FP32; all n elements. */
 int svbrdf_desc_feat_loss(const void* f, int dtypes, const void* t, const float* gram_grad, float coef, int mask,
                           void* g, float* partial, long long n, void* stream);
 

@@ -703,7 +703,7 @@ int svbrdf_desc_pool_bwd_loss(const void* gy, const void* x, const void* target,
 int svbrdf_desc_feat_loss(const void* f, int dtypes, const void* t, const float* gram_grad, float coef, int mask,
                           void* g, float* partial, long long n, void* stream) {
   if (!f || !t || n < 1) return fail(SVBRDF_ERR_INVALID, "null pointer or empty");
-  if (dtypes < 0 || dtypes > 3) return fail(SVBRDF_ERR_INVALID, "feat_loss: dtypes must be 0..3");
+  if (dtypes < 0 || dtypes > 3) dtypes = 1;  // the flag that the argument was: any non-zero value, f BF16
   cudaStream_t st = (cudaStream_t)stream;
   const bool wide = n % 8 == 0 && (((uintptr_t)f | (uintptr_t)t | (uintptr_t)gram_grad | (uintptr_t)g) & 15) == 0;
 #define SVB_FL(TF, TT, WIDE)                                                                        \

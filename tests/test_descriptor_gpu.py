@@ -602,3 +602,19 @@ def test_renders_of_other_shapes_than_the_targets(svb, cuda, mode):
     if mode == "reference":
         assert torch.equal(d.loss_and_grad(cur[:2])[2], first.loss_and_grad(cur[:2])[2])
     assert d.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flag", [4, 255, -1])
+def test_feature_loss_takes_other_nonzero_flags(svb, cuda, flag):
+    """The types' argument was a flag (any non-zero value: BF16 features, FP32 targets) before it
+    told the targets' type too: values outside 0..3 still mean that."""
+    N, L = svb._native, svb._native.lib()
+    f = torch.randn(4096, device=cuda).to(torch.bfloat16)
+    t, g, p = torch.randn(4096, device=cuda), [], []
+    for d in (1, flag):
+        g.append(torch.empty(4096, device=cuda, dtype=torch.bfloat16))
+        p.append(torch.zeros(L.svbrdf_desc_partials(), device=cuda))
+        N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), d, t.data_ptr(), None, 0.7, 0, g[-1].data_ptr(),
+                                        p[-1].data_ptr(), 4096, N.stream_handle(cuda)))
+    assert torch.equal(*g) and torch.equal(*p)
