@@ -514,7 +514,10 @@ __global__ void __launch_bounds__(kLossSumThreads) desc_loss_sums_kernel(const f
   constexpr int kWarps = kLossSumThreads / 32, kU = 3;  // units of a warp in flight
   static_assert(kWarps == 32 && kMaxLossSegs <= kWarps, "one lane per warp's share, one warp per segment");
   __shared__ float2 share[kMaxLossSegs][kWarps];
+  __shared__ unsigned in_double[kMaxLossSegs];  // bit w: warp w's share of the segment is a double's bits
   __shared__ double total[kMaxLossSegs];
+  if (threadIdx.x < kMaxLossSegs) in_double[threadIdx.x] = 0u;
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   long long unit = warp;  // of this warp, counted from the start of segment k
   for (int k = 0; k < segs.n; ++k) {
@@ -536,6 +539,7 @@ __global__ void __launch_bounds__(kLossSumThreads) desc_loss_sums_kernel(const f
     }
     while (unit >= units + kWarps) unit -= kWarps;  // the first of its units past the segment's end
     unit -= units;
+    const float own = sk;
     float lo = 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -544,13 +548,24 @@ __global__ void __launch_bounds__(kLossSumThreads) desc_loss_sums_kernel(const f
       lo += bl + ((sk - (s - bb)) + (b - bb));
       sk = s;
     }
-    if (lane == 0) share[k][warp] = make_float2(sk, lo);
+    if (fabsf(sk) <= 3.402823466e+38f) {  // every lane holds the same sum
+      if (lane == 0) share[k][warp] = make_float2(sk, lo);
+    } else {
+      // lane totals whose sum FP32 does not hold, or an infinity or NaN among them: in double
+      double d = (double)own;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      if (lane == 0) {
+        share[k][warp] = make_float2(__int_as_float(__double2loint(d)), __int_as_float(__double2hiint(d)));
+        atomicOr(&in_double[k], 1u << warp);
+      }
+    }
   }
   __syncthreads();
   if (warp < segs.n) {
     const float2 sh = share[warp][lane];
-    // an infinite sum has no rounding error to add (it reads NaN)
-    double t = (double)sh.x + (fabsf(sh.x) <= 3.402823466e+38f ? (double)sh.y : 0.0);
+    double t = (in_double[warp] >> lane) & 1u ? __hiloint2double(__float_as_int(sh.y), __float_as_int(sh.x))
+                                              : (double)sh.x + (double)sh.y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) total[warp] = segs.w[warp] * t;

@@ -618,3 +618,25 @@ def test_feature_loss_takes_other_nonzero_flags(svb, cuda, flag):
         N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), d, t.data_ptr(), None, 0.7, 0, g[-1].data_ptr(),
                                         p[-1].data_ptr(), 4096, N.stream_handle(cuda)))
     assert torch.equal(*g) and torch.equal(*p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fill,want", [(1e38, 6.4e36), (float("inf"), float("inf")), (-float("inf"), -float("inf")),
+                                       (float("nan"), float("nan")), (None, float("nan"))])
+def test_loss_sums_beyond_fp32(svb, cuda, fill, want):
+    """Segments whose sum FP32 does not hold, though its weighted total does (FP64 totals: 1e-6), and
+    infinities and NaN, which stay what they are; None mixes both infinities. The other group is a
+    plain sum beside it."""
+    import ctypes
+    N, L = svb._native, svb._native.lib()
+    buf = torch.ones(1000, device=cuda)
+    buf[300:364] = float("inf") if fill is None else fill
+    if fill is None:
+        buf[310] = -float("inf")
+    out = torch.empty(2, device=cuda)
+    arr = [(ctypes.c_longlong * 2)(300, 364), (ctypes.c_longlong * 2)(64, 600), (ctypes.c_double * 2)(1e-3, 0.5),
+           (ctypes.c_int * 2)(0, 1)]
+    N.check(L.svbrdf_desc_loss_sums(buf.data_ptr(), 2, *[ctypes.addressof(a) for a in arr], out.data_ptr(),
+                                    N.stream_handle(cuda)))
+    got, want = out.cpu().double(), torch.tensor([want, 300.0], dtype=torch.float64)
+    assert torch.allclose(got, want, rtol=1e-6, atol=0.0, equal_nan=True)
