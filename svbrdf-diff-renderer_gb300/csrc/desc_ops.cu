@@ -441,7 +441,7 @@ desc_feat_loss_kernel(const TF* __restrict__ f, const TT* __restrict__ t, const 
                       float coef, int mask, __nv_bfloat16* __restrict__ g, float* __restrict__ partial, long long n) {
   __shared__ float s_red[kLossThreads / 32];
   constexpr int E = WIDE ? 8 : 1, U = 2;
-  float acc = 0.0f;
+  float acc[U] = {};  // one per step in flight, and a step's eight squares first among themselves
   const long long step = (long long)kLossBlocks * kLossThreads * E;
   for (long long i0 = (blockIdx.x * (long long)kLossThreads + threadIdx.x) * E; i0 < n; i0 += U * step) {
     float fv[U][E], tv[U][E], gg[U][E];
@@ -465,14 +465,15 @@ desc_feat_loss_kernel(const TF* __restrict__ f, const TT* __restrict__ t, const 
     for (int u = 0; u < U; ++u) {
       const long long i = i0 + u * step;
       if (i >= n) continue;
-      float gv[E];
+      float gv[E], sq = WIDE ? 0.0f : acc[u];
 #pragma unroll
       for (int e = 0; e < E; ++e) {
         const float d = fv[u][e] - tv[u][e];
-        acc = fmaf(d, d, acc);
+        sq = fmaf(d, d, sq);
         gv[e] = gram_grad ? fmaf(coef, d, gg[u][e]) : coef * d;
         if (mask && !(fv[u][e] > 0.0f)) gv[e] = 0.0f;
       }
+      acc[u] = WIDE ? acc[u] + sq : sq;
       if (!g) continue;
       if constexpr (WIDE) bf8_store(g + i, gv);
       else g[i] = __float2bfloat16_rn(gv[0]);
@@ -480,8 +481,10 @@ desc_feat_loss_kernel(const TF* __restrict__ f, const TT* __restrict__ t, const 
   }
   if (partial) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
+    for (int u = 1; u < U; ++u) acc[0] += acc[u];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc[0];
     __syncthreads();
     if (threadIdx.x == 0) {
       float s = 0.0f;

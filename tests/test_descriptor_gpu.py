@@ -640,3 +640,21 @@ def test_loss_sums_beyond_fp32(svb, cuda, fill, want):
                                     N.stream_handle(cuda)))
     got, want = out.cpu().double(), torch.tensor([want, 300.0], dtype=torch.float64)
     assert torch.allclose(got, want, rtol=1e-6, atol=0.0, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [0.93524, 1.40396, 1.3928, 0.63764])
+def test_feature_loss_sum_of_a_large_map(svb, cuda, d):
+    """The squared sum where a thread adds 64 equal terms, whose roundings all go one way: each
+    block's share within what eights of terms, two sums of four of them, one addition and the
+    block's eight warps may round off (4.5 + 2.5 + 1 + 4.4 units of 2^-24, every one at its worst).
+    One sum over all 64 is off by 16 units on these values."""
+    N, L = svb._native, svb._native.lib()
+    blocks = L.svbrdf_desc_partials()
+    n = blocks * 256 * 64
+    f, t = torch.full((n,), d, device=cuda), torch.zeros(n, device=cuda)
+    p = torch.zeros(blocks, device=cuda)
+    N.check(L.svbrdf_desc_feat_loss(f.data_ptr(), 0, t.data_ptr(), None, 0.0, 0, None, p.data_ptr(), n,
+                                    N.stream_handle(cuda)))
+    want = 256 * 64 * float(f[0]) ** 2
+    assert float((p.double() - want).abs().max()) <= 12.4 * 2.0 ** -24 * want
