@@ -117,6 +117,7 @@ desc_conv1_fwd_kernel(const float* __restrict__ r, const float* __restrict__ w, 
     if (more) fetch(y0 + kTileY);
     const int y = y0 + row, x = x0 + px0;
     const size_t pix = ((size_t)v * H + y) * W + x;
+    float sq_tile = 0.0f;  // a pixel's squares first, then a tile's: no sum of 128 terms in a row
     float4 tv[4];
     if (LOSS && y < H) {
 #pragma unroll
@@ -168,7 +169,7 @@ desc_conv1_fwd_kernel(const float* __restrict__ r, const float* __restrict__ w, 
           if (px + 4 < kPx && x + px + 4 < W)
             tv[px % 4] = __ldg(reinterpret_cast<const float4*>(target + (pix + px + 4) * 64) + cg);
           const float d0 = a0 - t4.x, d1 = a1 - t4.y, d2 = a2 - t4.z, d3 = a3 - t4.w;
-          sq = fmaf(d0, d0, fmaf(d1, d1, fmaf(d2, d2, fmaf(d3, d3, sq))));
+          sq_tile += fmaf(d0, d0, fmaf(d1, d1, fmaf(d2, d2, d3 * d3)));
           __nv_bfloat162 g0 = __floats2bfloat162_rn(coef * d0, coef * d1), g1 = __floats2bfloat162_rn(coef * d2, coef * d3);
           pk.x = *reinterpret_cast<uint32_t*>(&g0);
           pk.y = *reinterpret_cast<uint32_t*>(&g1);
@@ -176,6 +177,7 @@ desc_conv1_fwd_kernel(const float* __restrict__ r, const float* __restrict__ w, 
         }
       }
     }
+    sq += sq_tile;
     // buffer (rep + 1) & 1 was last read in the previous tile, before that tile's barrier
     if (more) stage((rep + 1) & 1, y0 + kTileY);
     __syncthreads();
@@ -371,6 +373,7 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
     for (int e = 0; e < 4; ++e) {  // channel pairs 2e, 2e + 1
       const float2 g = bf2f(gr, e);
       float2 xv[4];
+      float sq_pair = 0.0f;  // the pair's eight squares first
 #pragma unroll
       for (int k = 0; k < 4; ++k) xv[k] = bf2f(xr[k], e);
       int amx = 0, amy = 0;
@@ -387,8 +390,8 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
         float2 ad = bf2f(ar[k], e);
         if constexpr (LOSS) {
           const float2 d = make_float2(xv[k].x - ad.x, xv[k].y - ad.y);
-          sq = fmaf(d.x, d.x, sq);
-          sq = fmaf(d.y, d.y, sq);
+          sq_pair = fmaf(d.x, d.x, sq_pair);
+          sq_pair = fmaf(d.y, d.y, sq_pair);
           ad = __bfloat1622float2(__floats2bfloat162_rn(coef * d.x, coef * d.y));
         }
         float vx = AVG ? 0.25f * g.x : (amx == k ? g.x : 0.0f);
@@ -398,6 +401,7 @@ __global__ void __launch_bounds__(256) desc_pool_bwd_kernel(const __nv_bfloat16*
         const __nv_bfloat162 h = __floats2bfloat162_rn(xv[k].x > 0.0f ? vx : 0.0f, xv[k].y > 0.0f ? vy : 0.0f);
         reinterpret_cast<uint32_t*>(&o[k])[e] = *reinterpret_cast<const uint32_t*>(&h);
       }
+      if constexpr (LOSS) sq += sq_pair;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(gx + b0 + offs[k]) = o[k];

@@ -658,3 +658,23 @@ def test_feature_loss_sum_of_a_large_map(svb, cuda, d):
                                     N.stream_handle(cuda)))
     want = 256 * 64 * float(f[0]) ** 2
     assert float((p.double() - want).abs().max()) <= 12.4 * 2.0 ** -24 * want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [1.90244, 1.4486, 1.00592, 0.965])
+def test_conv1_feature_term_of_equal_features(svb, cuda, d):
+    """conv1_1's feature term where all 128 squares of a thread are equal (no weights, the bias is the
+    feature), so that their roundings all go one way: each block's share within what a pixel's
+    four, a tile's eight, a block's four tiles and eight warps may round off (2.3 + 4.4 + 2.3 + 4.4 units
+    of 2^-24, one more for a product). One sum over all 128 is off by 30 units on these values."""
+    N, L = svb._native, svb._native.lib()
+    v, h, w = 2, 32, 48
+    r = torch.rand(v, 3, h, w, device=cuda)
+    wt, b = torch.zeros(64, 3, 3, 3, device=cuda), torch.full((64,), d, device=cuda)
+    t = torch.zeros(v, h, w, 64, device=cuda)
+    y16, g = (torch.empty(v, h, w, 64, device=cuda, dtype=torch.bfloat16) for _ in range(2))
+    p = torch.zeros(L.svbrdf_desc_conv1_loss_partials(v, h, w), device=cuda)
+    N.check(L.svbrdf_desc_conv1_loss(r.data_ptr(), wt.data_ptr(), b.data_ptr(), y16.data_ptr(), v, h, w, 0,
+                                     t.data_ptr(), 0.37, g.data_ptr(), p.data_ptr(), N.stream_handle(cuda)))
+    want = t.numel() / p.numel() * float(b[0]) ** 2
+    assert float((p.double() - want).abs().max()) <= 14.4 * 2.0 ** -24 * want
