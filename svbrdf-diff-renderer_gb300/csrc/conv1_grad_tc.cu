@@ -108,13 +108,7 @@ conv1_grad_kernel(const __grid_constant__ CUtensorMap tmap_g, const __nv_bfloat1
           tma_4d(abase + (uint32_t)((s * NX + m) * kTileBytes), &tmap_g, 0, xw + 128 * m, ys - 1 + j, img, fb);
         ++issued;
       }
-      if (issued < n_rows) {  // aborted: let the copies in flight land before the block can exit
-        for (int j = issued > kStages ? issued - kStages : 0; j < issued; ++j) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&full_bar[j % kStages]), (uint32_t)(j / kStages) & 1u) && ++it < kSpin) {
-          }
-        }
-      }
+      drain_loads(full_bar, issued, kStages);
     }
   } else if (warp == 1) {
     if (lane == 0) {

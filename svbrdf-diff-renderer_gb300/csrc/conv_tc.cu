@@ -313,19 +313,8 @@ conv3x3_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           }
         }
       }
-      if (bad) {
-        // aborted: no load may still be writing shared memory when the CTA exits
-        for (int i = qa > AST ? qa - AST : 0; i < qa; ++i) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&afull[i % AST]), (uint32_t)(i / AST) & 1u) && ++it < kSpin) {
-          }
-        }
-        for (int i = qb > BST ? qb - BST : 0; i < qb; ++i) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&bfull[i % BST]), (uint32_t)(i / BST) & 1u) && ++it < kSpin) {
-          }
-        }
-      }
+      drain_loads(afull, qa, AST);
+      drain_loads(bfull, qb, BST);
     }
   } else if (warp == 1) {
     if (lane == 0) {

@@ -176,13 +176,7 @@ conv_tf32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
           ++q;
         }
       }
-      if (bad) {  // let the copies in flight land before the CTA can exit
-        for (int i = q > STAGES ? q - STAGES : 0; i < q; ++i) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&full_bar[i % STAGES]), (uint32_t)(i / STAGES) & 1u) && ++it < kSpin) {
-          }
-        }
-      }
+      drain_loads(full_bar, q, STAGES);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -384,18 +378,8 @@ conv_tf32_halo_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           }
         }
       }
-      if (bad) {  // let the copies in flight land before the CTA can exit
-        for (int i = qa > AST ? qa - AST : 0; i < qa; ++i) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&afull[i % AST]), (uint32_t)(i / AST) & 1u) && ++it < kSpin) {
-          }
-        }
-        for (int i = qb > BST ? qb - BST : 0; i < qb; ++i) {
-          uint32_t it = 0;
-          while (!mbar_try(smem_u32(&bfull[i % BST]), (uint32_t)(i / BST) & 1u) && ++it < kSpin) {
-          }
-        }
-      }
+      drain_loads(afull, qa, AST);
+      drain_loads(bfull, qb, BST);
     }
   } else if (warp == 1) {
     if (lane == 0) {

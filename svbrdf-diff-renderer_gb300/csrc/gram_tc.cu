@@ -53,15 +53,6 @@ __device__ __forceinline__ void release_tmem(uint64_t* acc_bar, uint32_t tmem, u
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
 
-// Aborted producer: wait (bounded) for the loads of the last min(issued, stages) stages to land.
-__device__ __forceinline__ void drain_loads(uint64_t* full_bar, int issued, int stages) {
-  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) {
-    uint32_t it = 0;
-    while (!mbar_try(smem_u32(&full_bar[i % stages]), (uint32_t)(i / stages) & 1u) && ++it < kSpin) {
-    }
-  }
-}
-
 // grid (tiles_i * tiles_j, splits, V). Rows of the partial at or beyond C are not stored.
 // Z64 (C = 64): a stage is the one 64-channel box, which is B and A's first atom; A's second
 // atom (rows 64..127, never stored) is a zero atom written once per CTA, reached through A's
@@ -134,7 +125,7 @@ gram_kernel(const __grid_constant__ CUtensorMap tmap_f, float* __restrict__ part
         for (int b = 0; b < BN / 64; ++b) tma_2d(st + A_BYTES + b * kAtom, &tmap_f, j0 + 64 * b, row, fb);
         ++issued;
       }
-      if (issued < steps) drain_loads(full_bar, issued, STAGES);
+      drain_loads(full_bar, issued, STAGES);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -302,7 +293,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         tma_2d(st + A_BYTES, &tmap_b, i * 64, b * Nn + n0, fb);
         ++issued;
       }
-      if (issued < steps) drain_loads(full_bar, issued, STAGES);
+      drain_loads(full_bar, issued, STAGES);
     }
   } else if (warp == 1) {
     if (lane == 0) {

@@ -47,6 +47,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
   }
   return true;
 }
+// The producer's last act: wait (bounded) for the loads of the last min(issued, stages) stages to
+// land, before the block's shared memory goes away. An MMA or epilogue warp that gave up leaves
+// loads behind also when the producer had issued its last one by then and saw no wait run out; in a
+// healthy launch they have landed or are about to be used.
+__device__ __forceinline__ void drain_loads(uint64_t* full_bar, int issued, int stages) {
+  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) {
+    uint32_t it = 0;
+    while (!mbar_try(smem_u32(&full_bar[i % stages]), (uint32_t)(i / stages) & 1u) && ++it < kSpin) {
+    }
+  }
+}
 __device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                        uint32_t bar) {
   asm volatile(

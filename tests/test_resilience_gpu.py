@@ -67,6 +67,41 @@ def test_launch_under_a_set_error_word_returns(svb, cuda, variant):
     assert all(torch.equal(x, y) for x, y in zip(runs[0].tex, runs[1].tex))
 
 
+@pytest.mark.parametrize("gram", [True, False])
+def test_tensor_core_launches_under_a_set_error_word_return(svb, cuda, gram):
+    """The waits of the tensor-core kernels may give up in any warp while the error word is set: the
+    launches wait for their loads, return and keep the code, and the next descriptor and
+    convolutions are healthy."""
+    N = svb._native
+    gen = torch.Generator().manual_seed(5)
+    tgt, cur = (torch.rand(2, 3, 256, 256, generator=gen).to(cuda) for _ in range(2))
+    make = lambda: svb.descriptor.VGGDescriptor(cuda, seed=2, mode="config" if gram else "reference")
+    d = make()
+    d.load(tgt)
+    d.err.fill_(41)
+    for _ in range(3):
+        d._loss_and_grad_eager(cur)
+    assert d.device_error() == 41
+    x, w = (torch.rand(*s, generator=gen).to(cuda) for s in ((2, 64, 64, 64), (64, 9 * 64)))
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    outs = []
+    for code in (41, 0, 0):
+        err.fill_(code)
+        y = torch.zeros_like(x)
+        N.check(N.lib().svbrdf_gen_conv_tf32(x.data_ptr(), w.data_ptr(), y.data_ptr(), 2, 64, 64, 64, 64, 3, 1,
+                                             err.data_ptr(), N.stream_handle(cuda)))
+        assert int(err.item()) == code
+        outs.append(y)
+    assert torch.equal(outs[1], outs[2]) and bool((outs[1] > 0).all())
+    runs = []
+    for _ in range(2):
+        e = make()
+        e.load(tgt)
+        runs.append(e._loss_and_grad_eager(cur))
+        assert e.device_error() == 0
+    assert all(torch.equal(a, b) and torch.isfinite(a).all() for a, b in zip(*runs))
+
+
 @pytest.mark.parametrize("ctas", [0, 5])
 @pytest.mark.parametrize("variant,light", [(2, True), (3, True), (2, False), (3, False)])
 def test_workspace_is_usable_again_once_the_word_is_zeroed(svb, cuda, variant, light, ctas):
