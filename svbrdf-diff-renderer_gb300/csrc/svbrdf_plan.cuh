@@ -58,7 +58,9 @@ struct __align__(16) MatDesc {
   double inv_n;       // 1 / (3 V H W)
 };
 
-constexpr int kPlanMagic = 0x53564232;  // "SVB2"
+// Another value with every change of the layout: a plan that another build made is refused, where its
+// offsets would be read as other ones.
+constexpr int kPlanMagic = 0x53564233;  // "SVB3"
 
 // Adam hyper-parameters of a batched launch; the step itself lives on the device so
 // one captured graph can be replayed indefinitely.

@@ -289,6 +289,24 @@ def test_corrupt_plan_is_rejected_on_host(svb, lib):
     assert lib.svbrdf_selftest_wait_timeout(fake, 16, 0, None) == -1
 
 
+def test_plan_of_another_layout_is_rejected_on_host(svb, lib):
+    """A plan with the mark of the layout before the runs of tiles were listed in it is refused: its
+    header has other fields at the offsets that the kernels would read."""
+    SV = svb._native
+    mats, keep = _materials(SV, [(64, 64, 9)])
+    cfg = SV.svbrdf_batch_config(480, 960, 3, 3)
+    n = lib.svbrdf_batched_plan_bytes(mats, 1, ctypes.byref(cfg))
+    buf = np.zeros(n, np.uint8)
+    assert lib.svbrdf_batched_plan(mats, 1, ctypes.byref(cfg), buf.ctypes.data, n) == 0
+    need = lib.svbrdf_batched_workspace_bytes(buf.ctypes.data)
+    assert need > 0
+    buf[0:4] = np.frombuffer(np.int32(0x53564232).tobytes(), np.uint8)
+    assert lib.svbrdf_batched_workspace_bytes(buf.ctypes.data) == 0
+    fake = ctypes.c_void_p(16)
+    assert lib.svbrdf_batched_steps(fake, buf.ctypes.data, 1, fake, 0.01, 0.9, 0.999, 1e-8, fake, 4, 3, fake, need,
+                                    None) == -1
+
+
 def test_texel_count_limit_rejected_on_host(lib):
     """H*W must stay below 2^31 (the kernels index texels in 64 bits, rows and columns in 32):
     the host rejects larger shapes before touching the device. Nothing is launched here."""
