@@ -926,6 +926,13 @@ __device__ __forceinline__ const float2* pair_acquire(RingCursor& rc, const floa
 // dynamic shared memory). P chunks carry the tile and its material, target chunks the views
 // of the chunk, so consumers read everything a tile needs from shared memory and never wait
 // on one another.
+// (material, first texel) of entry k of a texel-pair plan, whose entries are its tiles in order.
+__device__ __forceinline__ int2 seq_entry(const int4* seq, int k, int n_tiles) {
+  if (k >= n_tiles) return make_int2(-1, 0);
+  const int4 e = seq[k];
+  return make_int2(e.y, e.z);
+}
+
 struct __align__(16) PairSlotRec {
   float4 cxy[kPairChunkViews];  // target chunks: (cx, cx, cy, cy) of views 3c .. 3c+2
   float4 czz[kPairChunkViews];  // (cz, cz, 0, 0)
@@ -934,7 +941,7 @@ struct __align__(16) PairSlotRec {
   float* m1;
   float* m2;
   int run_tile, run_ends;       // the run's first tile; 1 if it ends here and another follows
-  int tile, first, W, H;        // ... tile id and first texel
+  int pad0, first, W, H;        // ... and first texel
   int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
   float P[4];                   // light power
@@ -989,7 +996,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
   bool ok = true;
   RingCursor rc{0, 0u, true};
   const int4* seq = (const int4*)(plan + hdr->off_seq);
-  const int4 sq_first = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
+  const int2 sq_first = seq_entry(seq, k0, n_tiles), sq_second = seq_entry(seq, k0 + 1, n_tiles);
   int cur = -1;  // the producer's staged material
 
   for (int it = 0; it < iters; ++it) {
@@ -997,19 +1004,20 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       // ------------------------------------------------------------ producer (the whole warp)
       // Lane 0 fills the slot's record and posts the chunk's bytes on its full barrier (a
       // release that publishes the record); lanes 0 .. nplanes-1 then issue one plane copy
-      // each. The next tile's entry is loaded one tile ahead and a material's fields and
-      // views only when the material changes.
-      int4 sq_next = sq_first;
+      // each. A tile ends where the next one starts, so its entry is loaded two tiles ahead; a
+      // material's fields and views only when the material changes.
+      int2 sq_next = sq_first, sq_after = sq_second;
       int run_tile = 0;
       for (int k = k0; k < k1 && ok; ++k) {
-        const int4 sq = sq_next;
-        if (k + 1 < n_tiles) sq_next = seq[k + 1];
-        if (sq.y != cur || k == k0) {
+        const int2 sq = sq_next;
+        sq_next = sq_after;
+        sq_after = seq_entry(seq, k + 2, n_tiles);
+        if (sq.x != cur || k == k0) {
           // the material's fields and views are staged still if the last iteration ended with it;
           // its light power may have been stepped since, by another CTA
-          const bool staged = sq.y == cur;
-          cur = sq.y;
-          run_tile = sq.x;
+          const bool staged = sq.x == cur;
+          cur = sq.x;
+          run_tile = k;
           __syncwarp();
           const MatDesc& m = mats[cur];
           if (!staged) {
@@ -1021,11 +1029,11 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
         }
         const MatDesc& md = s_prod_md;
         const int T = md.H * md.W, V = md.V;
-        const int first = sq.z;
+        const int first = sq.y;
         // the tile ends where the next one of its material starts
-        const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
+        const int count = (sq_next.x == cur ? sq_next.y : T) - first;
         const uint32_t bytes = (uint32_t)count * 4u;
-        const int run_ends = k + 1 < k1 && sq_next.y != cur;
+        const int run_ends = k + 1 < k1 && sq_next.x != cur;
         const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
         for (int q = 0; q < nt + 4; ++q) {
           if (issued >= R) {
@@ -1047,7 +1055,7 @@ batched_pair_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
             PairSlotRec& r = recs[slot];
             if (q == 0 || q >= nt + 1) {  // P, P', M and S chunks carry the tile record
               r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
-              r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
+              r.first = first; r.W = md.W; r.H = md.H;
               r.V = V; r.all_coloc = md.all_coloc; r.count = count;
               r.run_tile = run_tile; r.run_ends = run_ends;
               r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
@@ -1317,7 +1325,7 @@ struct __align__(16) FuseStateRec {
   float* m1;
   float* m2;
   int run_tile, run_ends;  // the run's first tile; 1 if it ends here and another follows
-  int tile, first, W, H;
+  int tile, first, W, H;  // tile: variant 4
   int V, all_coloc, count, pad1;  // count: the tile's texels
   float scale, size, inv_w, pad2;
   float P[4];
@@ -1403,14 +1411,18 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
     uint32_t phase = 0, sphase = 0;
     long long issued = 0, states = 0;
     bool ok = true;
-    int4 sq_next = k0 < k1 ? seq[k0] : make_int4(0, 0, 0, 0);
+    // A tile ends where the next one starts, so its entry is loaded two tiles ahead: one tile ahead,
+    // the load's latency stood before every tile's state copy (32 materials of 512^2, two iterations:
+    // 1207 us, two tiles ahead 1200).
+    int2 sq_next = seq_entry(seq, k0, n_tiles), sq_after = seq_entry(seq, k0 + 1, n_tiles);
     int cur = -1, run_tile = 0;
     for (int k = k0; k < k1 && ok; ++k) {
-      const int4 sq = sq_next;
-      if (k + 1 < n_tiles) sq_next = seq[k + 1];
-      if (sq.y != cur) {
-        cur = sq.y;
-        run_tile = sq.x;
+      const int2 sq = sq_next;
+      sq_next = sq_after;
+      sq_after = seq_entry(seq, k + 2, n_tiles);
+      if (sq.x != cur) {
+        cur = sq.x;
+        run_tile = k;
         __syncwarp();
         const MatDesc& m = mats[cur];
         if (lane == 0) s_prod_md = m;
@@ -1420,11 +1432,11 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       }
       const MatDesc& md = s_prod_md;
       const int T = md.H * md.W, V = md.V;
-      const int first = sq.z;
+      const int first = sq.y;
       // the tile ends where the next one of its material starts
-      const int count = (k + 1 < n_tiles && sq_next.y == cur ? sq_next.z : T) - first;
+      const int count = (sq_next.x == cur ? sq_next.y : T) - first;
       const uint32_t bytes = (uint32_t)count * 4u;
-      const int run_ends = k + 1 < k1 && sq_next.y != cur;
+      const int run_ends = k + 1 < k1 && sq_next.x != cur;
       const int nt = (V + kPairChunkViews - 1) / kPairChunkViews;
       // the state area is free once every consumer warp is done with the previous tile
       if (k > k0) {
@@ -1435,7 +1447,7 @@ batched_fuse_kernel(const char* __restrict__ plan, AdamHyper hyper, int* __restr
       if (lane == 0) {
         FuseStateRec& r = s_rec;
         r.tex = md.tex; r.m1 = md.m1; r.m2 = md.m2;
-        r.tile = sq.x; r.first = first; r.W = md.W; r.H = md.H;
+        r.first = first; r.W = md.W; r.H = md.H;
         r.V = V; r.all_coloc = md.all_coloc; r.count = count;
         r.run_tile = run_tile; r.run_ends = run_ends;
         r.scale = md.scale; r.size = md.size; r.inv_w = md.inv_w;
