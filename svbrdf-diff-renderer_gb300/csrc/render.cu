@@ -47,7 +47,8 @@ int device_sm_count() {
 // ------------------------------------------------------------------ kernels
 constexpr int kRenderThreads = 256;
 
-// Forward render with the image loss (Microfacet.render_loss), one texel per thread.
+// Forward render with the image loss (Microfacet.render_loss), one texel per thread; LOSS 0..2 (without a
+// loss render_texels_fwd_kernel runs).
 template <int LOSS>
 __global__ void __launch_bounds__(kRenderThreads)
 render_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, const float* __restrict__ lit,
@@ -82,10 +83,8 @@ render_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, 
     const long long vb = 3LL * V * T * b;
     for (int v = 0; v < V; ++v) {
       float io[3];
-      if (LOSS >= 0) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) io[c] = targets[vb + (3LL * v + c) * T + idx];
-      }
+      for (int c = 0; c < 3; ++c) io[c] = targets[vb + (3LL * v + c) * T + idx];
       if (s_views[v].coloc != 0.f)
         texel_view<kModeFwd, LOSS, false, true>(m, px, py, s_views[v], s_pow, io, loss, dummy);
       else
@@ -96,15 +95,13 @@ render_fwd_kernel(const float* __restrict__ tex, const float* __restrict__ cam, 
       }
     }
   }
-  if (LOSS >= 0) {
-    const float bl = block_sum<kRenderThreads>(loss, s_red);
-    if (publish_partial_and_check_last(partials, counter, make_float4(bl, 0.f, 0.f, 0.f), &s_flag)) {
-      double tot[4];
-      sum_partials<kRenderThreads>(partials, gridDim.x, tot, s_dred);
-      if (threadIdx.x == 0) {
-        *loss_out = (float)(tot[0] * inv_n);
-        *counter = 0u;
-      }
+  const float bl = block_sum<kRenderThreads>(loss, s_red);
+  if (publish_partial_and_check_last(partials, counter, make_float4(bl, 0.f, 0.f, 0.f), &s_flag)) {
+    double tot[4];
+    sum_partials<kRenderThreads>(partials, gridDim.x, tot, s_dred);
+    if (threadIdx.x == 0) {
+      *loss_out = (float)(tot[0] * inv_n);
+      *counter = 0u;
     }
   }
 }
