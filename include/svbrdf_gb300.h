@@ -492,9 +492,10 @@ int svbrdf_gen_conv_tf32_ex(const float* x, const float* weight, float* y, void*
 
 /* svbrdf_gen_conv_tf32_ex followed by the style layer's epilogue of svbrdf_gen_act_nhwc, or with s2
  * of svbrdf_gen_act_scale_nhwc, on its output: y receives the convolution (the adjoint reads it) and
- * out [b][ho][wo][cout] the activation. 3x3 convolutions of maps of 16 and more rows run both in one
- * kernel, with the same values. d [b][cout], noise [b][ho][wo] (with ns, one float) and s2 [b][cout]
- * may be NULL. */
+ * out [b][ho][wo][cout] the activation. A 3x3 convolution to a map of 16 and more rows and 8 and more
+ * columns that does not split K runs both in one kernel where d, bias, s2 and out are 16-byte
+ * aligned, any other the two kernels, with the same values. d [b][cout], noise [b][ho][wo] (with ns,
+ * one float) and s2 [b][cout] may be NULL. */
 int svbrdf_gen_conv_act_tf32(const float* x, const float* weight, float* y, void* ws, long long ws_bytes, int b,
                              int hin, int win, int cin, int cout, int ksize, int pad, const float* d,
                              const float* noise, const float* ns, const float* bias, float gain, const float* s2,

@@ -112,8 +112,8 @@ class BatchedOptim:
         return sum(H * W * (216 + 12 * V) for H, W, V, _ in self.meta)
 
     def launches(self, iters: int) -> int:
-        """Kernel launches ``iters`` iterations take with this plan's variant. With a learnable light
-        every iteration counts as one, although the texel-pair kernel runs up to FUSE_MAX of them
+        """Kernel launches that ``iters`` iterations take at most with this plan's variant. With a
+        learnable light every iteration counts as one, although variant 2 runs up to FUSE_MAX of them
         in one cooperative launch where the device holds its whole grid at once."""
         return -(-iters // FUSE_MAX) if self.config.variant >= 3 and not self.optim_light else iters
 

@@ -223,8 +223,8 @@ static int launch(const CUtensorMap& mg, const __nv_bfloat16* w16, const float* 
   }
   const int sms = device_sm_count();
   const int windows = w <= 128 * NX ? 1 : (w + 128 * NX - 3) / (128 * NX - 2);
-  // strips of equal height that make about two blocks per SM; each reads two rows more than it writes,
-  // so none is under 4 rows
+  // strips that make about two blocks per SM; each reads two rows more than it writes, so they have 4
+  // rows or more (a column's last one what is left)
   const long long total = (long long)n * windows * h, slots = 2LL * (sms > 0 ? sms : 1);
   long long rows = (total + slots - 1) / slots;
   rows = rows < 4 ? 4 : rows > h ? h : rows;

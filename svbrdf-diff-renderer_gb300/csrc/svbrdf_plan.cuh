@@ -7,9 +7,10 @@
 //   | int4 seq[n_tiles] (order[k]'s tile, material and first texel, in CTA order; a tile
 //     of variants 2 and 3 ends where its material's next one starts, the others have tile_texels texels)
 //   | variants 2 and 3: int run_tile[n_runs] | int cta_run[n_ctas+1] | int mat_run[n_mat+1]
-// Tiles of one material are contiguous in tile-index order (mat_tile_off), so each
-// material's loss is a fixed-order sum over a tile range. cta_off[c]..cta_off[c+1]
-// indexes `order`, the planner's balanced permutation of tile ids for CTA c.
+// Tiles of one material are contiguous in tile-index order (mat_tile_off), so each material's loss is a
+// fixed-order sum over a tile range, or in variants 2 and 3 over its runs: a run is a CTA's
+// consecutive tiles of one material, named by its first tile. cta_off[c]..cta_off[c+1] indexes
+// `order`, the tile ids of CTA c; `order` is the identity.
 #pragma once
 
 #include "svbrdf_math.cuh"
@@ -71,7 +72,8 @@ struct AdamHyper {
 // Workspace of a batched launch: [0] completion counter, [1] error word, [2] number of the last
 // iteration that a cooperative launch has finished (it only ever counts up), then from byte
 // 256 the per-(tile, warp) partial losses, then (plans with a learnable light) the
-// per-(tile, warp) partial light-power gradients, 3 floats each.
+// per-(tile, warp) partial light-power gradients, 3 floats each, then one total per tile and quantity.
+// Variants 2 and 3 use the slots of a run's first tile for the whole run.
 constexpr int kWsCounter = 0;
 constexpr int kWsError = 1;
 constexpr int kWsIteration = 2;
